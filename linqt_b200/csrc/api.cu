@@ -919,8 +919,8 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
   char *Ls = (char *)s->get("lr_L", blk * M);
   char *Rs = (char *)s->get("lr_R", blk * M);
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
-  double2 *raw = (double2 *)s->get("mu_raw", sizeof(double2) * (size_t)M * M);
-  LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * (size_t)M * M, s->stream));
+  double2 *raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * (size_t)M * M);  // hi, lo
+  LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * (size_t)M * M, s->stream));
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
     {
@@ -930,7 +930,7 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
     }
     {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw);
+      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + (size_t)M * M);
       ph.launches(2);
     }
   }
@@ -985,8 +985,8 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
   double2 *raw = nullptr, *acc = nullptr, *acc_c = nullptr;
   if (mu) {
-    raw = (double2 *)s->get("mu_raw", sizeof(double2) * (size_t)M * M);
-    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * (size_t)M * M, s->stream));
+    raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * (size_t)M * M);  // hi, lo
+    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * (size_t)M * M, s->stream));
   }
   if (out) {
     acc = (double2 *)s->get("kubo_acc", sizeof(double2) * 2 * (size_t)nump);
@@ -1002,7 +1002,7 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     }
     if (mu) {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw);
+      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + (size_t)M * M);
       ph.launches(2);
     }
     if (out) {

@@ -235,6 +235,7 @@ struct Session {
   long phase_launches[4] = {0, 0, 0, 0};
   int sm_count = 148;
   size_t hbm_budget = 0;  // chunking budget; 0 = what the device has free
+  size_t rns_budget = 8ull << 30;  // residue planes of the FP64 contraction (mu_rns.cu), at most
   bool barrier_used = false;  // a persistent kernel ran since the last error check
   // fault injection for tests (linqt_session_inject_barrier_timeout): grid barriers await
   // inject_extra more CTAs than launched and give up after inject_limit polls
@@ -304,8 +305,15 @@ void moments1d_from_dots(Session *s, const double2 *dots, int steps, int M, int 
 // mu_raw[M x M] += sum_k conj(L[m0][k]) * Rv[m1][k], FP64 (or FP32-input) operands
 // C(i,j) (+)= sum_k conj(A[i][k]) B[j][k], FP64
 void zgemm_cn(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, double2 *C, bool accumulate);
+// raw_lo takes the low parts of a contraction that gives more than FP64 (mu_rns.cu)
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw);
+                 double2 *mu_raw, double2 *raw_lo);
+// FP64 contraction in residues on the INT8 tensor cores (mu_rns.cu): device bytes of residue
+// planes it works in (0: this shape, or the memory left, is better served by the FP64 kernel)
+size_t rns_plane_bytes(Session *s, int MA, int MB, long K);
+size_t rns_bytes(int MA, int MB, long K);  // the planes of the whole product (0: the FP64 kernel's shape)
+void zgemm_cn_rns(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, size_t plane_bytes,
+                  double2 *raw_hi, double2 *raw_lo);
 void mu_finalize(Session *s, const double2 *mu_raw, int M, int R, double2 *mu);
 void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 *dst);
 // R random-phase states (R x N, state-major) from Philox4x32-10 with the given seed (states.cu)

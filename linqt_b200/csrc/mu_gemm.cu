@@ -6,6 +6,9 @@
 // Both operands are "K-major": moment m's block T_m is N*R contiguous complex
 // numbers, so K = N*R and the contraction also sums over the R random vectors.
 //
+// The large FP64 tables of the solves go to the residue kernel (mu_rns.cu: rns_bytes holds the
+// line and both sides' times); this one takes the rest, FP32 blocks and the energy sums.
+//
 // FP64 path: FP64 tensor-core MMA (mma.sync m8n8k4 f64; there is no FP64 tcgen05 kind)
 // on 64x64 complex output tiles per CTA (8 warps of 32x16), cp.async double-buffered
 // 16-deep K slices in padded shared memory (conflict-free fragment loads), split-K over
@@ -245,9 +248,12 @@ void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 
 }
 
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw) {
+                 double2 *mu_raw, double2 *raw_lo) {
   if (!fp32_inputs) {
-    zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
+    if (const size_t planes = rns_plane_bytes(s, M, M, K))
+      zgemm_cn_rns(s, (const double2 *)L, M, (const double2 *)Rv, M, K, planes, mu_raw, raw_lo);
+    else
+      zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
   } else if (i8_digits(precision)) {
     mu_contract_i8(s, L, Rv, M, K, i8_digits(precision), mu_raw);  // tcgen05 INT8 digits, exact sums (mu_i8.cu)
   } else if (precision == LINQT_PREC_MIXED_TF32 && mu_tc_supported(K)) {

@@ -51,6 +51,7 @@ struct Job {
   void *states = nullptr;  // pinned host copy (server pool); NULL: generated on the device
   size_t states_cap = 0;
   size_t footprint = 0;
+  size_t rns_budget = 0;  // residue planes of the FP64 contraction, part of the footprint
   int block_width = 1;
   int status = 0;  // 0 pending, 1 running, 2 done, <0 error
   bool alone = false;  // ran out of memory next to other requests: runs again with none beside it
@@ -206,6 +207,7 @@ struct linqt_server {
           const int n = H.n, R = job->req.R, M = job->req.M;
           const size_t sb = sizeof(double2) * (size_t)R * n;
           const size_t mb = sizeof(double2) * (size_t)M * (job->req.kind == LINQT_REQ_DOS ? 1 : M);
+          s.rns_budget = job->rns_budget;
           s.hbm_budget = job->footprint;  // fixed per request: chunking independent of the other requests
           double2 *d_st = (double2 *)s.get("io_states", sb);
           double2 *d_mu = (double2 *)s.get("io_mu", mb);
@@ -319,6 +321,15 @@ int linqt_server_submit(linqt_server *srv, const linqt_request *req, long *ticke
     const int n = req->H->op.n;
     job->block_width = pick_width(*req, n, srv->sm_count, srv->budget);
     job->footprint = estimate_footprint(*req, n, srv->sm_count, job->block_width);
+    // planes for the FP64 contraction where the budget has room for them (else the request
+    // contracts without them)
+    if (req->kind == LINQT_REQ_KUBO_BASTIN && req->precision == LINQT_PREC_FP64) {
+      const size_t planes = std::min(rns_bytes(req->M, req->M, (long)n * job->block_width), (size_t)2 << 30);
+      if (job->footprint + planes <= srv->budget) {
+        job->rns_budget = planes;
+        job->footprint += planes;
+      }
+    }
     if (job->footprint > srv->budget)
       fail(LINQT_ERR_NOMEM, "server: request footprint " + std::to_string(job->footprint >> 20) +
                                 " MiB exceeds the HBM budget");
