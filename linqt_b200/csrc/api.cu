@@ -983,15 +983,34 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   char *Ls = (char *)s->get("lr_L", blk * M);
   char *Rs = (char *)s->get("lr_R", blk * M);
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
-  double2 *raw = nullptr, *acc = nullptr, *acc_c = nullptr;
+  double2 *raw = nullptr, *acc = nullptr, *acc_c = nullptr, *tab = nullptr;
+  const size_t MM = (size_t)M * M;
   if (mu) {
-    raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * (size_t)M * M);  // hi, lo
-    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * (size_t)M * M, s->stream));
+    raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * MM);  // hi, lo
+    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * MM, s->stream));
   }
+  // sigma's site sums: from the raw table in double-double (kubo_table.cu), once per solve, or from
+  // the transforms of every site (kubo_fft.cu), by the times both take at these sizes; the FP64
+  // moments need the same table, so there only what the residues cost beyond the FP64 kernel
+  // (0.9 ps per value of K and 64 x 64 tile) counts
+  size_t planes = 0;
   if (out) {
+    const long K = (long)N * ch.Rc;
+    const double tiles = (M + 63) / 64, f64_us = 75 + 9.0e-4 * tiles * tiles * K;
+    double extra_us = rns_us(M, K);
+    if (mu && !fp32) extra_us = rns_faster(M, M, K) ? 0 : std::max(0.0, extra_us - f64_us);
+    if (kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
+      planes = rns_plane_bytes(s, M, M, K);
     acc = (double2 *)s->get("kubo_acc", sizeof(double2) * 2 * (size_t)nump);
-    LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
-    acc_c = (double2 *)s->get("kubo_acc_c", sizeof(double2) * 2 * (size_t)nump);
+    if (!planes) {
+      LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
+      acc_c = (double2 *)s->get("kubo_acc_c", sizeof(double2) * 2 * (size_t)nump);
+    } else if (mu && !fp32) {
+      tab = raw;
+    } else {
+      tab = (double2 *)s->get("kubo_tab", sizeof(double2) * 2 * MM);
+      LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
+    }
   }
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
@@ -1002,15 +1021,25 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     }
     if (mu) {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + (size_t)M * M);
+      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + MM, fp32 ? 0 : planes);
       ph.launches(2);
     }
-    if (out) {
+    if (out && !(tab && tab == raw)) {
       PhaseScope ph(s, PH_FFT);
-      kubo_fft_sites(s, Ls, Rs, (long)N * ch.Rc, M, nump, formula, fp32, acc_c);
-      add_into(s, acc, acc_c, 2 * nump);
-      ph.launches(4);
+      if (tab) {
+        zgemm_cn_rns(s, Ls, M, Rs, M, (long)N * ch.Rc, fp32, planes, tab, tab + MM);
+        ph.launches(3);
+      } else {
+        kubo_fft_sites(s, Ls, Rs, (long)N * ch.Rc, M, nump, formula, fp32, acc_c);
+        add_into(s, acc, acc_c, 2 * nump);
+        ph.launches(4);
+      }
     }
+  }
+  if (tab) {
+    PhaseScope ph(s, PH_FFT);
+    kubo_table_sums(s, tab, tab + MM, M, nump, formula, acc);
+    ph.launches(5);
   }
   PhaseScope ph(s, PH_OTHER);
   if (mu) mu_finalize(s, raw, M, R, mu);

@@ -305,15 +305,20 @@ void moments1d_from_dots(Session *s, const double2 *dots, int steps, int M, int 
 // mu_raw[M x M] += sum_k conj(L[m0][k]) * Rv[m1][k], FP64 (or FP32-input) operands
 // C(i,j) (+)= sum_k conj(A[i][k]) B[j][k], FP64
 void zgemm_cn(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, double2 *C, bool accumulate);
-// raw_lo takes the low parts of a contraction that gives more than FP64 (mu_rns.cu)
+// raw_lo takes the low parts of a contraction that gives more than FP64 (mu_rns.cu); with
+// planes > 0 an FP64 contraction goes there whatever its shape
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw, double2 *raw_lo);
-// FP64 contraction in residues on the INT8 tensor cores (mu_rns.cu): device bytes of residue
-// planes it works in (0: this shape, or the memory left, is better served by the FP64 kernel)
+                 double2 *mu_raw, double2 *raw_lo, size_t planes = 0);
+// Contraction in residues on the INT8 tensor cores, exact up to the 53-bit rounding of its inputs
+// (mu_rns.cu).  rns_faster: whether an FP64 product is faster there; rns_us: its time;
+// rns_bytes: the planes of the whole product; rns_plane_bytes: the planes it gets (0: memory is
+// short, use the FP64 kernel).
+bool rns_faster(int MA, int MB, long K);
+double rns_us(int M, long K);
+size_t rns_bytes(int MA, int MB, long K);
 size_t rns_plane_bytes(Session *s, int MA, int MB, long K);
-size_t rns_bytes(int MA, int MB, long K);  // the planes of the whole product (0: the FP64 kernel's shape)
-void zgemm_cn_rns(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, size_t plane_bytes,
-                  double2 *raw_hi, double2 *raw_lo);
+void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
+                  size_t plane_bytes, double2 *raw_hi, double2 *raw_lo);
 void mu_finalize(Session *s, const double2 *mu_raw, int M, int R, double2 *mu);
 void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 *dst);
 // R random-phase states (R x N, state-major) from Philox4x32-10 with the given seed (states.cu)
@@ -347,6 +352,11 @@ inline size_t i8_digit_bytes(int digits, int M, long K) {
 void kubo_prefactors(Session *s, int M, int nump, double2 *pf);
 void kubo_fft_sites(Session *s, const void *L, const void *Rv, long nsites, int M, int nump, int formula,
                     bool fp32_inputs, double2 *acc);
+// the same from the raw moment table hi + lo (kubo_table.cu); its time, and that of the site
+// transforms of one call (us)
+void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc);
+double kubo_table_us(int M, int nump, int formula);
+double kubo_sites_us(long nsites, int M, int nump, int formula);
 void kubo_postprocess(Session *s, const double2 *acc, int R, int nump, int formula, int N, double band_width,
                       double band_center, double *out);
 

@@ -13,6 +13,9 @@
 // and ket_m = R_m[l] (= OPR T_m(H) phi).  Products of the transforms are summed over
 // sites into p[k] (and w[k]).
 //
+// These kernels serve solves with few sites, or few sites per energy; larger ones take the sums from
+// the moment table (kubo_table.cu), by the times of kubo_sites_us and kubo_table_us.
+//
 // Design: one CTA per site at a time (persistent, the CTAs interleaved over the sites),
 // all 8 (or 4) transforms of the site in shared memory.  nump = 16 * 16 * R3,
 // R3 in {1, 2, 4, 8}: pass 1 does 16-point DFTs in registers straight from the
@@ -524,13 +527,16 @@ void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump
   LQ_LAUNCHED();
 }
 
+bool shared_memory_fft(int nump, int formula) {
+  const bool pow2 = nump >= 256 && nump <= 2048 && (nump & (nump - 1)) == 0;
+  return pow2 && (formula == LINQT_KUBO_BASTIN ? nump <= 1024 : true);
+}
+
 template <class Tin>
 void kubo_fft_sites_t(Session *s, const Tin *L, const Tin *Rv, long nsites, int M, int nump, int formula,
                       const double2 *pf, double2 *acc) {
   const bool bastin = formula == LINQT_KUBO_BASTIN;
-  const bool pow2 = nump >= 256 && nump <= 2048 && (nump & (nump - 1)) == 0;
-  const bool fits = pow2 && (bastin ? nump <= 1024 : true);
-  if (fits) {
+  if (shared_memory_fft(nump, formula)) {
     switch (nump) {
       case 256: bastin ? launch_fft<1, 8>(s, L, Rv, nsites, M, pf, acc) : launch_fft<1, 4>(s, L, Rv, nsites, M, pf, acc); return;
       case 512: bastin ? launch_fft<2, 8>(s, L, Rv, nsites, M, pf, acc) : launch_fft<2, 4>(s, L, Rv, nsites, M, pf, acc); return;
@@ -545,6 +551,16 @@ void kubo_fft_sites_t(Session *s, const Tin *L, const Tin *Rv, long nsites, int 
 }
 
 }  // namespace
+
+// Measured on one B200: 32.6 ns a site at 1024 energies for Bastin (8 transforms; Greenwood has 4);
+// the direct transforms 0.51 fs per site, moment, energy and transform.  Direct transforms of
+// more moments than their shared memory holds are refused: no time, so that they stay so.
+double kubo_sites_us(long nsites, int M, int nump, int formula) {
+  const double seqs = formula == LINQT_KUBO_BASTIN ? 8 : 4;
+  if (shared_memory_fft(nump, formula)) return 20 + nsites * (double)nump * seqs * 4.0e-6;
+  if (sizeof(double2) * 2 * (size_t)M > 227 * 1024) return 0;
+  return 20 + nsites * (double)nump * M * seqs * 5.1e-7;
+}
 
 void kubo_prefactors(Session *s, int M, int nump, double2 *pf) {
   k_prefactors<<<(M + 255) / 256, 256, 0, s->stream>>>(M, nump, pf);

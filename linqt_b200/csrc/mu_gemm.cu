@@ -6,7 +6,7 @@
 // Both operands are "K-major": moment m's block T_m is N*R contiguous complex
 // numbers, so K = N*R and the contraction also sums over the R random vectors.
 //
-// The large FP64 tables of the solves go to the residue kernel (mu_rns.cu: rns_bytes holds the
+// The large FP64 tables of the solves go to the residue kernel (mu_rns.cu: rns_faster holds the
 // line and both sides' times); this one takes the rest, FP32 blocks and the energy sums.
 //
 // FP64 path: FP64 tensor-core MMA (mma.sync m8n8k4 f64; there is no FP64 tcgen05 kind)
@@ -248,10 +248,11 @@ void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 
 }
 
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw, double2 *raw_lo) {
+                 double2 *mu_raw, double2 *raw_lo, size_t planes) {
   if (!fp32_inputs) {
-    if (const size_t planes = rns_plane_bytes(s, M, M, K))
-      zgemm_cn_rns(s, (const double2 *)L, M, (const double2 *)Rv, M, K, planes, mu_raw, raw_lo);
+    if (!planes && rns_faster(M, M, K)) planes = rns_plane_bytes(s, M, M, K);
+    if (planes)
+      zgemm_cn_rns(s, L, M, Rv, M, K, false, planes, mu_raw, raw_lo);
     else
       zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
   } else if (i8_digits(precision)) {

@@ -1,6 +1,6 @@
 // FP64 moment contraction on the INT8 tensor cores, exact in a residue number system.
 //
-//   raw(m0, m1) += sum_k conj(L[m0][k]) * Rv[m1][k]          (FP64 Chebyshev blocks)
+//   raw(m0, m1) += sum_k conj(L[m0][k]) * Rv[m1][k]     (FP64 or FP32 Chebyshev blocks)
 //
 // The FP64 tensor-core rate of the B200 is its FP64 FMA rate (36 TFLOP/s), a hundredth of its
 // INT8 rate, so the product is taken in integers (the modular form of the Ozaki scheme:
@@ -35,6 +35,7 @@
 
 #include <cstdint>
 
+#include "dd.cuh"
 #include "internal.cuh"
 #include "tc_common.cuh"
 
@@ -138,8 +139,9 @@ __device__ __forceinline__ uint32_t low_bytes(int a, int b, int c, int d) {
 // multiply-add r = X - p q on the low words; per complex and modulus two small reductions
 // of r_a + s r_b and r_a - s r_b (below 2^14: a 21-bit reciprocal is enough for
 // |residue| <= p/2 + 1).
+template <class Tc>
 __global__ void __launch_bounds__(256, 2)
-    k_residues(const double2 *__restrict__ srcA, const double2 *__restrict__ srcB, long ld, long K, int kc, int rows_a,
+    k_residues(const Tc *__restrict__ srcA, const Tc *__restrict__ srcB, long ld, long K, int kc, int rows_a,
                int rows_b, int nkb, int8_t *__restrict__ plA, int8_t *__restrict__ plB, int *__restrict__ expA,
                int *__restrict__ expB, int nchunk) {
   __shared__ unsigned red[8];
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(256, 2)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long k0 = (long)c * kc;
   const int len = (int)min((long)kc, K - k0);  // complex values of this chunk
-  const double2 *x = (b_side ? srcB : srcA) + (size_t)row * ld + k0;
+  const Tc *x = (b_side ? srcB : srcA) + (size_t)row * ld + k0;
   const int base = blockIdx.x * kPart;
   double2 v[4][4];
   unsigned mx = 0;
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(256, 2)
     const int k = base + (g * 8 + warp) * kBk + lane * 4;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      v[g][q] = k + q < len ? __ldg(x + k + q) : make_double2(0.0, 0.0);
+      v[g][q] = k + q < len ? to_d2(__ldg(x + k + q)) : make_double2(0.0, 0.0);
       mx = max(mx, max((unsigned)__double2hiint(v[g][q].x) & 0x7fffffffu,
                        (unsigned)__double2hiint(v[g][q].y) & 0x7fffffffu));
     }
@@ -468,29 +470,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRnsThreads, 1)
 // ---------------------------------------------------------------------------
 // Chinese remainders
 // ---------------------------------------------------------------------------
-// s + e = a + b exactly (Knuth's two-sum)
-__device__ __forceinline__ void two_sum(double a, double b, double &s, double &e) {
-  s = a + b;
-  const double t = s - a;
-  e = (a - (s - t)) + (b - t);
-}
-// (hi, lo) += (h, l)
-__device__ __forceinline__ void dd_add(double &hi, double &lo, double h, double l) {
-  double s, e;
-  two_sum(hi, h, s, e);
-  e += lo + l;
-  two_sum(s, e, hi, lo);
-}
-// X 2^ex as hi + lo: three pieces of at most 48 bits, each exact in FP64
-__device__ __forceinline__ void dd_from_i128(__int128 X, int ex, double &hi, double &lo) {
+// X 2^ex in double-double: three pieces of at most 48 bits, each exact in FP64
+__device__ __forceinline__ double2 dd_from_i128(__int128 X, int ex) {
   const unsigned long long mask = (1ull << 48) - 1;
   const double a = (double)(long long)(X >> 96), b = (double)((unsigned long long)(X >> 48) & mask),
                c = (double)((unsigned long long)X & mask);
-  double s, e;
-  two_sum(a * 79228162514264337593543950336.0, b * 281474976710656.0, s, e);
-  dd_add(s, e, c, 0.0);
-  hi = ldexp(s, ex);
-  lo = ldexp(e, ex);
+  double2 v;
+  two_sum(a * 79228162514264337593543950336.0, b * 281474976710656.0, v.x, v.y);
+  v = dd_add(v, make_double2(c, 0.0));
+  return make_double2(ldexp(v.x, ex), ldexp(v.y, ex));
 }
 
 // raw(i, j) += sum over chunks of 2^(ea + eb - 106) X, X the integer with the residues of the
@@ -502,11 +490,12 @@ __global__ void __launch_bounds__(256)
   const size_t plane = (size_t)MA * pitch;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < (long)MA * MB; t += (long)gridDim.x * blockDim.x) {
     const int i = (int)(t / MB), j = (int)(t % MB);
-    double2 hi = raw_hi[t], lo = raw_lo[t];
+    const double2 hi = raw_hi[t], lo = raw_lo[t];
+    double2 re = make_double2(hi.x, lo.x), im = make_double2(hi.y, lo.y);
     for (int c = 0; c < nchunk; ++c) {
       const int ea = expA[(size_t)i * nchunk + c], eb = expB[(size_t)j * nchunk + c];
       if (ea == kBadExp || eb == kBadExp) {
-        hi.x = hi.y = __longlong_as_double(0x7ff8000000000000ll);
+        re.x = im.x = __longlong_as_double(0x7ff8000000000000ll);
         continue;
       }
       const uint8_t *r = res + (size_t)c * kPlanes * plane + (size_t)i * pitch + j;
@@ -528,14 +517,11 @@ __global__ void __launch_bounds__(256)
       // S = X + k P with |X| < P / 4 (modulo 2^128: X itself fits)
       const __int128 xr = (__int128)(sr - P * (u128)(unsigned)__float2int_rn(fr));
       const __int128 xi = (__int128)(si - P * (u128)(unsigned)__float2int_rn(fi));
-      double h, l;
-      dd_from_i128(xr, ea + eb - 106, h, l);
-      dd_add(hi.x, lo.x, h, l);
-      dd_from_i128(xi, ea + eb - 106, h, l);
-      dd_add(hi.y, lo.y, h, l);
+      re = dd_add(re, dd_from_i128(xr, ea + eb - 106));
+      im = dd_add(im, dd_from_i128(xi, ea + eb - 106));
     }
-    raw_hi[t] = hi;
-    raw_lo[t] = lo;
+    raw_hi[t] = make_double2(re.x, im.x);
+    raw_lo[t] = make_double2(re.y, im.y);
   }
 }
 
@@ -555,7 +541,7 @@ CUtensorMap make_map_rns(const void *base, int rows, long blocks) {
 
 }  // namespace
 
-// Which kernel contracts an MA x MB x K product, and the planes' bytes when it is this one.
+// Which kernel contracts an MA x MB x K product.
 // The line, from both sides measured on one B200 (contraction phase, this kernel / mu_gemm.cu, us):
 //   M = 1024, K = 65536: 3840 / 15165;  512, 65536: 1463 / 3832;  256, 65536: 680 / 870;
 //   160, 65536: 434 / 514;  128, 65536: 365 / 274;  64, 65536: 248 / 152: below 160 rows the
@@ -564,17 +550,26 @@ CUtensorMap make_map_rns(const void *base, int rows, long blocks) {
 //   by the serial K loop there;
 //   1024, 512: 171 / 147;  768, 512: 113 / 83;  512, 512: 63 / 79: K < M is bound by the
 //   residue tables (34 bytes per entry and chunk).
-size_t rns_bytes(int MA, int MB, long K) {
+bool rns_faster(int MA, int MB, long K) {
   const int m = std::min(MA, MB);
-  const bool use = m >= 160 ? K >= std::max(192, std::max(MA, MB)) : m >= 8 && K >= 192 && K <= 8192;
-  if (!use) return 0;
+  return m >= 160 ? K >= std::max(192, std::max(MA, MB)) : m >= 8 && K >= 192 && K <= 8192;
+}
+
+size_t rns_bytes(int MA, int MB, long K) {
   const size_t per_k = (size_t)kPlanes * (MA + MB);
   return per_k * (size_t)((K + kBk - 1) / kBk + K / kChunkMax + 1) * kBk;  // chunks are rounded up
 }
 
+// Time of the contraction here, us: 30 of launches, 13.5 ps an entry for the residues, the GEMMs of
+// the padded tiles at 2.4 POPS (fits the times above within 20 % at K >= 2048).
+double rns_us(int M, long K) {
+  const double tiles = (M + kRnsTile - 1) / kRnsTile, pad = tiles * kRnsTile;
+  return 30 + 2.0 * M * K * 13.5e-6 + kPlanes * pad * pad * K * 2 / 2.4e9;
+}
+
+// Planes for a contraction here, allocated (0: not enough memory is left).
 size_t rns_plane_bytes(Session *s, int MA, int MB, long K) {
   const size_t all = rns_bytes(MA, MB, K);
-  if (!all) return 0;
   const size_t per_k = (size_t)kPlanes * (MA + MB);
   const size_t least = per_k * (size_t)std::min(kPart, (int)((K + kBk - 1) / kBk) * kBk);
   size_t want = std::min(s->rns_budget, all);
@@ -587,15 +582,16 @@ size_t rns_plane_bytes(Session *s, int MA, int MB, long K) {
       return want;
     } catch (const Error &e) {
       if (e.code != LINQT_ERR_NOMEM) throw;
+      s->rns_budget = want / 2;  // do not ask for as much again on every call
     }
   }
   return 0;
 }
 
-// raw (hi + lo, MA x MB) += sum_k conj(A[i][k]) B[j][k], k < K, rows ld complex apart, with the
-// planes of at most plane_bytes bytes at a time.
-void zgemm_cn_rns(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, size_t plane_bytes,
-                  double2 *raw_hi, double2 *raw_lo) {
+// raw (hi + lo, MA x MB) += sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K),
+// with planes of at most plane_bytes bytes at a time.
+void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
+                  size_t plane_bytes, double2 *raw_hi, double2 *raw_lo) {
   // K chunks of equal length, a multiple of the GEMM block, short enough for one set of planes
   const size_t per_k = (size_t)kPlanes * (MA + MB);
   long cap = std::min<long>(kChunkMax, (long)(plane_bytes / per_k) / kBk * kBk);
@@ -631,7 +627,12 @@ void zgemm_cn_rns(Session *s, const double2 *A, int MA, const double2 *B, int MB
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    LQ_CUDA(cudaLaunchKernelEx(&cfg, k_residues, A + k0, B + k0, K, len, kc, MA, MB, nkb, plA, plB, eA, eB, nc));
+    if (fp32_inputs)
+      LQ_CUDA(cudaLaunchKernelEx(&cfg, k_residues<float2>, (const float2 *)A + k0, (const float2 *)B + k0, K, len, kc,
+                                 MA, MB, nkb, plA, plB, eA, eB, nc));
+    else
+      LQ_CUDA(cudaLaunchKernelEx(&cfg, k_residues<double2>, (const double2 *)A + k0, (const double2 *)B + k0, K, len,
+                                 kc, MA, MB, nkb, plA, plB, eA, eB, nc));
     const long tiles = (long)((MA + kRnsTile - 1) / kRnsTile) * ((MB + kRnsTile - 1) / kRnsTile) * kPlanes * nc;
     const int pairs = (int)std::max(1L, std::min(tiles, (long)s->sm_count / 2));
     k_rns_gemm<<<2 * pairs, kRnsThreads, smem, s->stream>>>(ta, tb, MA, MB, len, kc, nkb, nc, res, pitch, err);

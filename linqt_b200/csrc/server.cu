@@ -51,7 +51,7 @@ struct Job {
   void *states = nullptr;  // pinned host copy (server pool); NULL: generated on the device
   size_t states_cap = 0;
   size_t footprint = 0;
-  size_t rns_budget = 0;  // residue planes of the FP64 contraction, part of the footprint
+  size_t rns_budget = 0;  // residue planes, part of the footprint
   int block_width = 1;
   int status = 0;  // 0 pending, 1 running, 2 done, <0 error
   bool alone = false;  // ran out of memory next to other requests: runs again with none beside it
@@ -321,13 +321,14 @@ int linqt_server_submit(linqt_server *srv, const linqt_request *req, long *ticke
     const int n = req->H->op.n;
     job->block_width = pick_width(*req, n, srv->sm_count, srv->budget);
     job->footprint = estimate_footprint(*req, n, srv->sm_count, job->block_width);
-    // planes for the FP64 contraction where the budget has room for them (else the request
-    // contracts without them)
-    if (req->kind == LINQT_REQ_KUBO_BASTIN && req->precision == LINQT_PREC_FP64) {
+    // planes for the contraction in residues (the FP64 moments', and sigma's) where the budget
+    // has room for them and for the tables of sigma; else the request runs without them
+    if (req->kind == LINQT_REQ_KUBO_BASTIN && (req->precision == LINQT_PREC_FP64 || req->sigma_out)) {
       const size_t planes = std::min(rns_bytes(req->M, req->M, (long)n * job->block_width), (size_t)2 << 30);
-      if (job->footprint + planes <= srv->budget) {
+      const size_t tables = sizeof(double2) * 8 * (size_t)req->M * req->M;
+      if (job->footprint + planes + tables <= srv->budget) {
         job->rns_budget = planes;
-        job->footprint += planes;
+        job->footprint += planes + tables;
       }
     }
     if (job->footprint > srv->budget)
