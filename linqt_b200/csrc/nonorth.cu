@@ -117,7 +117,7 @@ __device__ void grid_totals(const double2 *part, int nv, int Rb, double2 *tot) {
 // partial sums -> barrier -> totals; false if the barrier gave up
 __device__ bool reduce(const NonOrthArgs &a, const double2 *vals, int nv, double2 *tot) {
   cta_partials(vals, nv, a.part, a.Rb);
-  if (!grid_barrier(a.bar, gridDim.x)) return false;
+  if (!grid_barrier(a.bar)) return false;
   grid_totals(a.part, nv, a.Rb, tot);
   return true;
 }
@@ -204,7 +204,7 @@ __device__ bool bicgstab(const NonOrthArgs &a, const double2 *b, double2 *x, Col
       const double2 beta = cmul(cdiv(s.rho, s.rho_old), cdiv(s.alpha, s.w));
       LQ_ELEMS { a.P[e] = cadd(a.R[e], cmul(beta, csub(a.P[e], cmul(s.w, a.V[e])))); }
     }
-    if (!grid_barrier(a.bar, gridDim.x)) return false;
+    if (!grid_barrier(a.bar)) return false;
     // v = S D^-1 p; <r0, v>
     {
       double2 q = make_double2(0, 0);
@@ -286,6 +286,7 @@ __device__ bool bicgstab(const NonOrthArgs &a, const double2 *b, double2 *x, Col
 __global__ void __launch_bounds__(kT) k_nonorth_1d(NonOrthArgs a) {
   __shared__ Col col[kMaxCols];
   __shared__ double2 tot[3 * kMaxCols];
+  grid_init(a.bar, gridDim.x);
   const int Rb = a.Rb, c = threadIdx.x % Rb;
   const long ne = (long)a.n * Rb, stride = (long)gridDim.x * kT;
   if ((int)threadIdx.x < Rb) col[threadIdx.x].total_it = 0;
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(kT) k_nonorth_1d(NonOrthArgs a) {
   if (a.OP.rp) {
     if (!bicgstab(a, a.phi, a.X, col, tot, make_double2(0, 0), -1)) return;
     LQ_ELEMS { T0[e] = gather(a.OP, (int)(e / Rb), c, Rb, a.X); }
-    if (!grid_barrier(a.bar, gridDim.x)) return;
+    if (!grid_barrier(a.bar)) return;
   } else {
     if (!bicgstab(a, a.phi, T0, col, tot, make_double2(0, 0), -1)) return;
   }
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kT) k_nonorth_1d(NonOrthArgs a) {
       a.B[e] = gather(a.H, (int)(e / Rb), c, Rb, Tm);
       dq = cfma_conj(a.phi[e], Tm[e], dq);
     }
-    if (!grid_barrier(a.bar, gridDim.x)) return;
+    if (!grid_barrier(a.bar)) return;
     if (m == 0) {  // T_1 = S^-1 H T_0
       if (!bicgstab(a, a.B, T1, col, tot, dq, 0)) return;
       continue;
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(kT) k_nonorth_1d(NonOrthArgs a) {
     double2 *t = T0;
     T0 = T1;
     T1 = t;
-    if (!grid_barrier(a.bar, gridDim.x)) return;
+    if (!grid_barrier(a.bar)) return;
   }
   if (blockIdx.x == 0 && (int)threadIdx.x < Rb) a.iters[threadIdx.x] = col[threadIdx.x].total_it;
 }

@@ -33,13 +33,20 @@ namespace linqt {
 namespace {
 
 constexpr int kThreads = 256;
+// Columns per thread up to which the 1D kernels load a row's own vectors before its gathers: one
+// L2 latency of a step instead of three (square 256 x 256, one vector: 1449 -> 1272 us for
+// 512 steps).  In k_recur_lr the same costs 2-3 % on blocks beyond L1 (registers) and is not done.
+constexpr int kHoist = 1;
 
 using Barrier = GridBarrier;
 
-template <class C>
-__device__ __forceinline__ C ldv(const C *p) {
-  return __ldca(p);
+// CTAs an SM holds: the gathers are latency-bound, so the registers of more columns per thread
+// are bounded (spills included) to keep the warps that hide it.
+template <class T>
+constexpr int min_ctas_1d(int vpt) {
+  return vpt <= 4 ? 4 : sizeof(T) == 4 ? 3 : 2;
 }
+constexpr int min_ctas_lr(int vpt) { return vpt <= 2 ? 4 : vpt == 4 ? 2 : 1; }
 
 // The V adjacent complex values a thread owns in a block row, loaded through L1 with the
 // widest aligned accesses (p is aligned to min(32, V * sizeof(C)) bytes: rows hold a power
@@ -199,7 +206,7 @@ __device__ size_t cache_rows(const int *__restrict__ rp, const int *__restrict__
 //   R (!HAS_V): Rst[0] given (phi); in place like L.
 // ---------------------------------------------------------------------------
 template <class T, int TPR, int VPT, bool HAS_V>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, min_ctas_lr(VPT))
     k_recur_lr(int n, const int *rp, const int *ci, const double2 *hv, const int *vrp, const int *vci,
                const double2 *vv, typename cplx_t<T>::type *Lst,
                typename cplx_t<T>::type *Rst, const typename cplx_t<T>::type *phi, typename cplx_t<T>::type *tb, int M,
@@ -223,6 +230,7 @@ __global__ void __launch_bounds__(kThreads)
   // neighbours (read by nearby tiles at about the same time) are still in L2.
   const int rfirst = cache ? r0 : blockIdx.x * gpb, rend = cache ? r1 : n;
   const int rstep = cache ? gpb : gridDim.x * gpb;
+  grid_init(bar, gridDim.x);
   for (int m = 0; m < M; ++m) {
     const bool doL = m + 1 < M;
     const C *xL = Lst + (size_t)m * blk;
@@ -302,7 +310,7 @@ __global__ void __launch_bounds__(kThreads)
         st_row<VPT>(yR + base, o);
       }
     }
-    if (m + 1 < M && !grid_barrier(bar, gridDim.x)) return;
+    if (m + 1 < M && !grid_barrier(bar)) return;
   }
 }
 
@@ -314,7 +322,7 @@ __global__ void __launch_bounds__(kThreads)
 // partials: [steps][grid][2] per-CTA sums.
 // ---------------------------------------------------------------------------
 template <class T, class HV, int TPR, int VPT, bool STACKED>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, min_ctas_1d<T>(VPT))
     k_recur_1d(int n, const int *rp, const int *ci, const HV *hv, const typename cplx_t<T>::type *phi, typename cplx_t<T>::type *x0, typename cplx_t<T>::type *b1,
                int steps, int M, int mode, double2 *__restrict__ partials, Barrier *bar, int cache,
                const int *__restrict__ sperm, const int *__restrict__ soff, int sC, long vstride, int nreal,
@@ -341,6 +349,7 @@ __global__ void __launch_bounds__(kThreads)
   }
   const int rfirst = cache ? r0 : bl * gpb, rend = cache ? r1 : n;  // as in k_recur_lr
   const int rstep = cache ? gpb : G1 * gpb;
+  grid_init(bar, gridDim.x);
   C *prev = nullptr, *cur = x0;
   for (int s = 0; s < steps; ++s) {
     const bool need_y = mode == 2 ? (2 * s + 1 < M) : (s + 1 < M);
@@ -353,11 +362,23 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int u = 0; u < VPT; ++u) acc[u] = make_double2(0, 0);
       const size_t base = (size_t)row * ldx + coff + c0;
-      if (prev) prefetch_l2(prev + base);  // T_{s-1} of this row, read after the gathers
+      // The row's own T_{s-1}, T_s and (mode 1) phi.  One or two columns per thread: loaded
+      // before the gathers, one L2 latency for all.  More columns would hold too many
+      // registers meanwhile: only asked for in L2, and loaded after the gathers.
+      C pv[VPT], xv[VPT], fv[VPT];
+      if constexpr (VPT <= kHoist) {
+        if (prev) ld_row<VPT>(prev + base, pv);
+        ld_row<VPT>(cur + base, xv);
+        if (mode == 1) ld_row<VPT>(phi + base, fv);
+      } else {
+        if (prev) prefetch_l2(prev + base);
+      }
 #pragma unroll 4
       for (int k = b; k < e; k += st) gather_fma<C, VPT>(to_d2(hv[k]), cur + (size_t)ci[k] * ldx + coff + c0, acc);
-      C pv[VPT], yv[VPT], xv[VPT];
-      if (prev) ld_row<VPT>(prev + base, pv);
+      C yv[VPT];
+      if constexpr (VPT > kHoist) {
+        if (prev) ld_row<VPT>(prev + base, pv);
+      }
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
         double2 ya = acc[u];
@@ -369,10 +390,9 @@ __global__ void __launch_bounds__(kThreads)
         yv[u] = from_d2<C>(ya);  // the value stored and used in the dot products
       }
       if (y) st_row<VPT>(y + base, yv);
-      ld_row<VPT>(cur + base, xv);
+      if constexpr (VPT > kHoist) ld_row<VPT>(cur + base, xv);
       if (mode == 1) {
-        C fv[VPT];
-        ld_row<VPT>(phi + base, fv);
+        if constexpr (VPT > kHoist) ld_row<VPT>(phi + base, fv);
 #pragma unroll
         for (int u = 0; u < VPT; ++u) d0 = cfma_conj(to_d2(fv[u]), to_d2(xv[u]), d0);
       } else {
@@ -384,13 +404,15 @@ __global__ void __launch_bounds__(kThreads)
         }
       }
     }
+    // the dot products' sums run while the other CTAs arrive
+    if (need_y) grid_arrive(bar);
     block_sum2(d0, d1);
     if (threadIdx.x == 0) {
       partials[((size_t)s * gridDim.x + blockIdx.x) * 2] = d0;
       partials[((size_t)s * gridDim.x + blockIdx.x) * 2 + 1] = d1;
     }
     if (!need_y) break;
-    if (!grid_barrier(bar, gridDim.x)) return;
+    if (!grid_wait(bar)) return;
     prev = cur;
     cur = y;
   }
@@ -403,7 +425,7 @@ __global__ void __launch_bounds__(kThreads)
 // over T_{s-1}; X accumulates coef[s] T_s as each T_s is produced (FP64).
 // ---------------------------------------------------------------------------
 template <int TPR, int VPT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, VPT <= 2 ? 4 : VPT == 4 ? 3 : 2)
     k_cheb_series(int n, const int *rp, const int *ci, const double2 *hv, double2 *X, double2 *a, double2 *b,
                   const double2 *__restrict__ coef, int K, Barrier *bar, int cache) {
   constexpr int RW = TPR * VPT;
@@ -427,30 +449,40 @@ __global__ void __launch_bounds__(kThreads)
       a[idx] = x;
       X[idx] = cmul(coef0, x);
     }
+  grid_init(bar, gridDim.x);
   double2 *prev = nullptr, *cur = a;
   for (int s = 1; s < K; ++s) {
-    if (!grid_barrier(bar, gridDim.x)) return;
+    if (!grid_barrier(bar)) return;
     double2 *y = prev ? prev : b;
     const double2 cs = coef[s];
     for (int pos = rfirst + threadIdx.x / TPR; pos < rend; pos += rstep) {
-      double2 acc[VPT];
+      double2 acc[VPT], pv[VPT], xv[VPT];
 #pragma unroll
       for (int u = 0; u < VPT; ++u) acc[u] = make_double2(0, 0);
+      const size_t base = (size_t)pos * RW + c0;
+      if constexpr (VPT <= kHoist) {  // before the gathers, as in k_recur_1d
+        if (prev) ld_row<VPT>(prev + base, pv);
+#pragma unroll
+        for (int u = 0; u < VPT; ++u) xv[u] = X[base + u];
+      }
       const int kb = rp[pos], ke = rp[pos + 1];
 #pragma unroll 4
       for (int k = kb; k < ke; ++k) gather_fma<double2, VPT>(hv[k], cur + (size_t)ci[k] * RW + c0, acc);
+      if constexpr (VPT > kHoist) {
+        if (prev) ld_row<VPT>(prev + base, pv);
+#pragma unroll
+        for (int u = 0; u < VPT; ++u) xv[u] = X[base + u];
+      }
 #pragma unroll
       for (int u = 0; u < VPT; ++u) {
-        const size_t idx = (size_t)pos * RW + c0 + u;
-        double2 yn = acc[u];
         if (prev) {
-          const double2 p = ldv(prev + idx);
-          yn.x = 2 * yn.x - p.x;
-          yn.y = 2 * yn.y - p.y;
+          acc[u].x = 2 * acc[u].x - pv[u].x;
+          acc[u].y = 2 * acc[u].y - pv[u].y;
         }
-        y[idx] = yn;
-        X[idx] = cadd(X[idx], cmul(cs, yn));  // X rows are this thread's own: no barrier needed
+        xv[u] = cadd(xv[u], cmul(cs, acc[u]));  // X rows are this thread's own: no barrier needed
       }
+      st_row<VPT>(y + base, acc);
+      st_row<VPT>(X + base, xv);
     }
     prev = cur;
     cur = y;
