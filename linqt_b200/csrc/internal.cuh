@@ -128,6 +128,33 @@ __device__ __forceinline__ float2 from_d2<float2>(double2 v) {
   return make_float2((float)v.x, (float)v.y);
 }
 
+// Sum of v over the threads before this one in the CTA (a multiple of 32 threads, at most 1024),
+// always in the same order.
+__device__ inline double exclusive_prefix(double v) {
+  __shared__ double warp_sum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double incl = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_sum[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    double s = lane < nw ? warp_sum[lane] : 0.0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    warp_sum[lane] = s;
+  }
+  __syncthreads();
+  const double before = __shfl_up_sync(0xffffffffu, incl, 1);
+  const double base = w ? warp_sum[w - 1] : 0.0;
+  __syncthreads();  // warp_sum may be used again
+  return lane ? base + before : base;
+}
+
 // ---------------------------------------------------------------------------
 // device operator: Hermitian-expanded CSR (plus optional FP32 copy and SELL-C)
 // ---------------------------------------------------------------------------

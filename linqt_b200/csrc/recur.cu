@@ -489,26 +489,29 @@ __global__ void __launch_bounds__(kThreads, VPT <= 2 ? 4 : VPT == 4 ? 3 : 2)
   }
 }
 
-// dots[2s + i] = sum_b partials[s][b][i]  (fixed order)
-__global__ void k_reduce_step_partials(const double2 *__restrict__ partials, int steps, int nb,
+// dots[(r*steps + s)*2 + i] = sum over the CTAs b of realisation r (b in [r*g1, (r+1)*g1); one
+// realisation: all) of partials[s][b][i].  One warp per (r, s), lanes striding over the CTAs, then a
+// fixed tree; with one thread per sum the loads of 256 to 592 CTAs one after the other took
+// 71 to 145 us.
+__global__ void k_reduce_step_partials(const double2 *__restrict__ partials, int steps, int nb, int g1, int nreal,
                                        double2 *__restrict__ dots) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * steps; t += gridDim.x * blockDim.x) {
-    const int s = t >> 1, i = t & 1;
-    double2 acc = make_double2(0, 0);
-    for (int b = 0; b < nb; ++b) acc = cadd(acc, partials[((size_t)s * nb + b) * 2 + i]);
-    dots[t] = acc;
-  }
-}
-
-// Stacked realisations: dots[(r*steps + s)*2 + i] = sum over the CTAs b of group r
-// (b in [r*g1, (r+1)*g1)) of partials[s][b][i]  (fixed order)
-__global__ void k_reduce_step_partials_split(const double2 *__restrict__ partials, int steps, int nb, int g1,
-                                             int nreal, double2 *__restrict__ dots) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * steps * nreal; t += gridDim.x * blockDim.x) {
-    const int i = t & 1, s = (t >> 1) % steps, r = (t >> 1) / steps;
-    double2 acc = make_double2(0, 0);
-    for (int b = r * g1; b < (r + 1) * g1; ++b) acc = cadd(acc, partials[((size_t)s * nb + b) * 2 + i]);
-    dots[t] = acc;
+  const int lane = threadIdx.x & 31;
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < steps * nreal; t += (gridDim.x * blockDim.x) >> 5) {
+    const int s = t % steps, r = t / steps;
+    double2 a0 = make_double2(0, 0), a1 = a0;
+    for (int b = r * g1 + lane; b < (r + 1) * g1; b += 32) {
+      const double2 *p = partials + ((size_t)s * nb + b) * 2;
+      a0 = cadd(a0, p[0]);
+      a1 = cadd(a1, p[1]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      a0 = cadd(a0, shfl_down2(a0, o));
+      a1 = cadd(a1, shfl_down2(a1, o));
+    }
+    if (lane == 0) {
+      dots[2 * (size_t)t] = a0;
+      dots[2 * (size_t)t + 1] = a1;
+    }
   }
 }
 
@@ -756,11 +759,9 @@ struct OneDF {
                     &M,        &mode,               &partials,    &bar,           &cache,      (void *)&sperm,
                     (void *)&soff, &sc, &vstride, &nreal, &ldx};
     coop_launch(s, f, grid, args, smem);
-    if (stacked)
-      k_reduce_step_partials_split<<<(2 * steps * nreal + 255) / 256, 256, 0, s->stream>>>(
-          partials, steps, grid, grid / nreal, nreal, dots);
-    else
-      k_reduce_step_partials<<<(2 * steps + 255) / 256, 256, 0, s->stream>>>(partials, steps, grid, dots);
+    const int groups = stacked ? nreal : 1;
+    k_reduce_step_partials<<<(steps * groups + 7) / 8, 256, 0, s->stream>>>(partials, steps, grid, grid / groups,
+                                                                           groups, dots);
     LQ_LAUNCHED();
   }
 };
