@@ -99,7 +99,7 @@ typedef struct linqt_opts {
                        value rounded once to FP32, products accumulated in FP64; every layout, persistent
                        recursion); other solvers accept 0 only */
   int thread_shape; /* 1D moments (linqt_moments1d[_dev]) in one persistent launch: 0 = the format's
-                       choice (shape 0, or autotuned with LINQT_FORMAT_AUTO); s + 1 = thread shape s,
+                       choice (by the block's size, or autotuned with LINQT_FORMAT_AUTO); s + 1 = thread shape s,
                        for tests and experiments (shape s of a block of R columns: min(R, 32) >> s
                        threads per row, at most 8 columns per thread; an invalid s is
                        LINQT_ERR_INVALID) */

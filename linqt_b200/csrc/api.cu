@@ -444,10 +444,10 @@ static void with_graph(Session *s, const linqt_opts &o, const std::string &key, 
 
 // ---------------------------------------------------------------------------
 // Sparse layout and thread shape of a persistent recursion.  LINQT_FORMAT_CSR: the
-// operator's CSR (whose per-CTA row slices the kernels keep in shared memory when they fit),
-// thread shape 0; LINQT_FORMAT_SELL: SELL-C-sigma with C = 32, shape 0; LINQT_FORMAT_LOCAL:
-// the CSR rows in the locality order (SELL with C = 1 over that order), shape 0;
-// LINQT_FORMAT_AUTO: the autotuner times a short run of the same recursion (trial(C, shape))
+// operator's CSR (whose per-CTA row slices the kernels keep in shared memory when they fit);
+// LINQT_FORMAT_SELL: SELL-C-sigma with C = 32; LINQT_FORMAT_LOCAL: the CSR rows in the locality
+// order (SELL with C = 1 over that order); all three with the thread shape `shape`
+// (recur_default_shape).  LINQT_FORMAT_AUTO: the autotuner times a short run of the same recursion (trial(C, shape))
 // for every layout (CSR cached, CSR uncached, SELL with C = 8 and 32, and on large blocks
 // the two locality layouts) and thread shape, keeps the fastest per
 // operator pair, block width and precision, and returns it.  Each candidate runs once
@@ -457,12 +457,12 @@ struct RecCfg {
   int sellC = 0, shape = 0;
 };
 
-static RecCfg pick_layout(Session *s, const DeviceOp &H, const std::string &key, int format, int Rc,
+static RecCfg pick_layout(Session *s, const DeviceOp &H, const std::string &key, int format, int Rc, int shape,
                           const std::function<void(int, int)> &trial, float *best_ms = nullptr) {
   if (best_ms) *best_ms = -1;
-  if (format == LINQT_FORMAT_CSR) return RecCfg{0, 0};
+  if (format == LINQT_FORMAT_CSR) return RecCfg{0, shape};
   if (format == LINQT_FORMAT_SELL || format == LINQT_FORMAT_LOCAL) {
-    return RecCfg{format == LINQT_FORMAT_SELL ? 32 : 1 | kSellLocality, 0};
+    return RecCfg{format == LINQT_FORMAT_SELL ? 32 : 1 | kSellLocality, shape};
   }
   DeviceOp &Hm = const_cast<DeviceOp &>(H);
   {
@@ -532,13 +532,16 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
   char *T = (char *)s->get("m1_T", 3 * esz * (size_t)N * Rc);
   PhaseScope ph(s, PH_RECURSION);
   long launches = 0;
+  const auto shape_of = [&](int w) {
+    return recur_default_shape((long)N * w, w, fp32, o.format == LINQT_FORMAT_LOCAL);
+  };
   // layout and thread shape for block width w, from short trials on the first w vectors
   auto tune = [&](int w, float *best_ms) {
     const size_t bw = esz * (size_t)N * w;
     const int Mt = std::min(M, 32), st = doubling ? (Mt + 1) / 2 : Mt;
     double2 *tdots = (double2 *)s->get("m1_trial_dots", sizeof(double2) * 2 * (size_t)st);
     return pick_layout(
-        s, H, layout_key(c64 ? "1d64" : "1d", op, w, fp32), o.format, w,
+        s, H, layout_key(c64 ? "1d64" : "1d", op, w, fp32), o.format, w, shape_of(w),
         [&](int C, int shape) {
           // a short recursion on the first chunk (the real run below starts from scratch)
           void *b0 = T, *b1 = T + bw, *b2 = T + 2 * bw;
@@ -696,7 +699,8 @@ static void realisations_stacked(Session *s, const DeviceOp *const *Hs, int S, c
     PhaseScope ph(s, PH_RECURSION);
     chunk_block(s, states, N, R, 0, R, phi, fp32);
     LQ_CUDA(cudaMemcpyAsync(b0, phi, blk, cudaMemcpyDeviceToDevice, s->stream));
-    recur_1d(s, H0, phi, b0, b1, steps, M, 2, R, fp32, dots, 0, 0, vals, S, c64);
+    recur_1d(s, H0, phi, b0, b1, steps, M, 2, R, fp32, dots, 0, recur_default_shape((long)N * R, Rs, fp32, false), vals, S,
+             c64);
     ph.launches(3);
   }
   PhaseScope p3(s, PH_OTHER);
@@ -796,7 +800,8 @@ static long lr_vectors(Session *s, const DeviceOp &H, const DeviceOp *opl, const
         LQ_CUDA(cudaMemcpyAsync(Lstore, phi, blk, cudaMemcpyDeviceToDevice, s->stream));
       if (!opr) LQ_CUDA(cudaMemcpyAsync(Rstore, phi, blk, cudaMemcpyDeviceToDevice, s->stream));
     };
-    const RecCfg cfg = pick_layout(s, H, layout_key("lr", opr, Rc, fp32), format, Rc, [&](int C, int shape) {
+    const RecCfg cfg = pick_layout(s, H, layout_key("lr", opr, Rc, fp32), format, Rc,
+                                   recur_lr_default_shape((long)H.n * Rc, Rc, fp32), [&](int C, int shape) {
       start();
       recur_lr(s, H, opr, Lstore, Rstore, phi, tmp3, std::min(M, 16), Rc, fp32, C, shape);
     });
@@ -1108,7 +1113,8 @@ static void moments_td_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, c
           spmm(s, *opr, make_double2(1, 0), PR, make_double2(0, 0), X0, Rc, false);
         else
           LQ_CUDA(cudaMemcpyAsync(X0, PR, blk, cudaMemcpyDeviceToDevice, s->stream));
-        recur_1d(s, H, PL, X0, X1, M, M, 1, Rc, false, dots + ((size_t)t * nchunks + ch) * 2 * M, sellC);
+        recur_1d(s, H, PL, X0, X1, M, M, 1, Rc, false, dots + ((size_t)t * nchunks + ch) * 2 * M, sellC,
+                 recur_default_shape((long)N * Rc, Rc, false, o.format == LINQT_FORMAT_LOCAL));
         if (t + 1 < NT) {  // the reference also evolves after the last step; nothing reads that
           cheb_series(s, H, PL, X0, X1, coef, (int)c.size(), Rc);
           cheb_series(s, H, PR, X0, X1, coef, (int)c.size(), Rc);

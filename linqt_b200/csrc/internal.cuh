@@ -425,6 +425,9 @@ void moments1d_from_dots_stream(cudaStream_t st, const double2 *dots, int steps,
 // without the cache; sellC > 0: its SELL-C-sigma layout with slice height sellC.
 // shape < recur_shapes(R): thread shape (shape s: min(R, 32) >> s threads per row)
 int recur_shapes(int R);
+// the shapes the recursions use when nothing else chooses one (items = values of a block)
+int recur_default_shape(long items, int R, bool fp32, bool locality);
+int recur_lr_default_shape(long items, int R, bool fp32);
 void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, void *Rstore, const void *phi,
               void *tbuf, int M, int R, bool fp32, int sellC, int shape = 0);
 // stacked != NULL: nreal realisations sharing H's pattern, values [nreal][nnz]; realisation r

@@ -836,6 +836,35 @@ int recur_shapes(int R) {
   }
 }
 
+namespace {
+// the narrowest shape with at least `want` columns per thread
+int shape_with(int R, int want) {
+  int s = 0;
+  while (s + 1 < recur_shapes(R) && R / std::max(1, std::min(R, 32) >> s) < want) ++s;
+  return s;
+}
+}  // namespace
+
+// Columns per thread.  While every thread has at most one item (a grid holds 592 x 256 = 152k
+// threads) one column is the shortest step; beyond, a thread's passes are dependent loads one
+// after the other, and 32-byte accesses (two FP64 or four FP32 columns) halve or quarter them.
+// Measured, us per step with 1, 2 and 4 columns: square 4096 sites x 16 vectors FP64 (66k values)
+// 3.3, 3.7, 4.7; honeycomb 8192 x 16 (131k) 4.1, 3.8, 4.6; cubic 10^6 x 32 571, 398, 530; FP32:
+// Kane-Mele 16384 x 16 (262k) 8.0, 6.6, 7.5; cubic 64000 x 8 (512k) 9.9, 7.6, 7.2; cubic 10^6 x
+// 32 562, 346, 267.  SELL and the complex64 operators alike (cubic 262144 x 16 FP32: 151, 73, 52
+// and 56, 45, 38); the locality order's narrow FP64 blocks keep one (cubic 262144 x 4: 22.8, 24.9).
+int recur_default_shape(long items, int R, bool fp32, bool locality) {
+  if (items <= 100000 || (locality && !fp32 && R < 8)) return 0;
+  return shape_with(R, fp32 && items > 400000 ? 4 : 2);
+}
+
+// The L/R kernel holds twice the sums: FP64 blocks keep shape 0 (Kane-Mele 16384 x 32: 22.2 us with
+// one column, 25.7 with two); large FP32 ones take four columns (Kane-Mele 65536 x 32: 81.6, 88.8
+// and 75.2; honeycomb 131072 x 32: 95.2, 106.0 and 85.3; 8192 x 32: 7.5, 8.1 and 6.6).
+int recur_lr_default_shape(long items, int R, bool fp32) {
+  return fp32 && items > 200000 ? shape_with(R, 4) : 0;
+}
+
 void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, void *Rstore, const void *phi,
               void *tbuf, int M, int R, bool fp32, int sellC, int shape) {
   const size_t blk = (size_t)H.n * R;
