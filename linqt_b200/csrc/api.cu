@@ -617,7 +617,8 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
         }
         x0 = b0;
       }
-      recur_1d(s, H, phi, x0, b1, steps, M, doubling ? 2 : 1, Rc, fp32, cd, cfg.sellC, cfg.shape, nullptr, 1, c64);
+      recur_1d(s, H, phi, x0, b1, steps, M, doubling ? 2 : 1, Rc, fp32, cd, cfg.sellC, cfg.shape, nullptr, 1, c64,
+               o.thread_shape == 0);
       launches += 2;
       continue;
     }

@@ -433,11 +433,20 @@ void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, vo
 // stacked != NULL: nreal realisations sharing H's pattern, values [nreal][nnz]; realisation r
 // owns columns [r R/nreal, (r+1) R/nreal), served by its own group of CTAs, and dots becomes
 // [nreal][steps][2]
+// on_chip: small lattices may run in one cluster (recur_cluster.cu), where shape has no meaning
 // c64: the operator's complex64 value copy (FP32 values, FP64 accumulation); CSR layouts only,
 // and `stacked` then holds float2 values
 void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
               bool fp32, double2 *dots, int sellC, int shape = 0, const void *stacked = nullptr, int nreal = 1,
-              bool c64 = false);
+              bool c64 = false, bool on_chip = true);
+// dots[(r*steps + s)*2 + i] = sums of partials[steps][nb][2] over the nb / nreal CTAs of each realisation
+void reduce_step_partials(Session *s, const double2 *partials, int steps, int nb, int nreal, double2 *dots);
+// the same recursions of small lattices in one cluster (recur_cluster.cu); false: too large
+bool cluster_recur_1d(Session *s, const DeviceOp &H, const void *phi, const void *x0, int steps, int M, int mode, int R,
+                      bool fp32, double2 *dots);
+bool cluster_recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lst, void *Rst, const void *phi, int M,
+                      int R, bool fp32);
+bool cluster_cheb_series(Session *s, const DeviceOp &H, void *X, const double2 *coef, int K, int R);
 // X <- sum_{s<K} coef[s] T_s(H) X on an FP64 block of R columns (a, b: scratch blocks), one
 // persistent launch (recur.cu)
 void cheb_series(Session *s, const DeviceOp &H, void *X, void *a, void *b, const double2 *coef, int K, int R);

@@ -515,6 +515,15 @@ __global__ void k_reduce_step_partials(const double2 *__restrict__ partials, int
   }
 }
 
+}  // namespace
+
+void reduce_step_partials(Session *s, const double2 *partials, int steps, int nb, int nreal, double2 *dots) {
+  k_reduce_step_partials<<<(steps * nreal + 7) / 8, 256, 0, s->stream>>>(partials, steps, nb, nb / nreal, nreal, dots);
+  LQ_LAUNCHED();
+}
+
+namespace {
+
 // Largest contiguous row slice (entries of one or two operators) a CTA owns for a given grid.
 size_t max_slice_bytes(const DeviceOp &H, const DeviceOp *V, int grid, size_t esz) {
   const int n = H.n;
@@ -759,10 +768,7 @@ struct OneDF {
                     &M,        &mode,               &partials,    &bar,           &cache,      (void *)&sperm,
                     (void *)&soff, &sc, &vstride, &nreal, &ldx};
     coop_launch(s, f, grid, args, smem);
-    const int groups = stacked ? nreal : 1;
-    k_reduce_step_partials<<<(steps * groups + 7) / 8, 256, 0, s->stream>>>(partials, steps, grid, grid / groups,
-                                                                           groups, dots);
-    LQ_LAUNCHED();
+    reduce_step_partials(s, partials, steps, grid, stacked ? nreal : 1, dots);
   }
 };
 
@@ -868,6 +874,7 @@ int recur_lr_default_shape(long items, int R, bool fp32) {
 void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, void *Rstore, const void *phi,
               void *tbuf, int M, int R, bool fp32, int sellC, int shape) {
   const size_t blk = (size_t)H.n * R;
+  if (sellC == 0 && cluster_recur_lr(s, H, V, Lstore, Rstore, phi, M, R, fp32)) return;
   Barrier *bar = barrier_for(s);
   if (fp32)
     dispatch<float, LRF>(R, shape, s, H, V, Lstore, Rstore, phi, tbuf, M, blk, bar, sellC);
@@ -877,7 +884,9 @@ void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, vo
 }
 
 void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
-              bool fp32, double2 *dots, int sellC, int shape, const void *stacked, int nreal, bool c64) {
+              bool fp32, double2 *dots, int sellC, int shape, const void *stacked, int nreal, bool c64,
+              bool on_chip) {
+  if (on_chip && sellC == 0 && !stacked && !c64 && cluster_recur_1d(s, H, phi, x0, steps, M, mode, R, fp32, dots)) return;
   Barrier *bar = barrier_for(s);
   const int Rw = stacked ? R / nreal : R;  // columns per CTA
   if (fp32)
@@ -888,6 +897,7 @@ void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1
 
 void cheb_series(Session *s, const DeviceOp &H, void *X, void *a, void *b, const double2 *coef, int K, int R) {
   LQ_REQUIRE(K >= 1, "Chebyshev series: at least one term");
+  if (cluster_cheb_series(s, H, X, coef, K, R)) return;
   Barrier *bar = barrier_for(s);
   dispatch<double, SeriesF>(R, 0, s, H, X, a, b, coef, K, bar);
   LQ_LAUNCHED();
