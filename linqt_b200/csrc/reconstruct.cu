@@ -57,7 +57,8 @@ __global__ void k_dos(const double2 *__restrict__ mu, int M, double N, double a,
 // kuboGreenwoodFromChebmom{,_FFTgrid}, kuboBastin{I,II,Sea,Surf}FromChebmom) on a
 // Jackson-damped table mu[M0][M1]:  kernel(x) = pref * sum_{m0,m1} f(x, m0, m1, mu).
 // Each is evaluated as Y(i, m0) = sum_m1 B(x_i, m1) mu(m0, m1) (an FP64 GEMM against a
-// coefficient table) and a per-energy sum over m0 with the left coefficient.  The
+// coefficient table) and a per-energy sum over m0 with the left coefficient, in the GEMM's epilogue
+// but for Bastin II.  The
 // coefficient functions are those of include/chebyshev_coefficients.hpp:9-32:
 //   delta(x, m)  = cos(m acos x) / f0 / pi,            f0 = sqrt(1 - x^2)
 //   G(x, m)      = -i (x - i f0)^m / f0,                (x - i f0)^m = exp(-i m acos x)
@@ -73,59 +74,181 @@ __device__ __host__ inline double grid_energy(int grid, int i, int n, double xbo
   return cos(M_PI * (2 * i + 0.5) / n);
 }
 
-__device__ inline double2 coef(int kind, double x, int m) {
-  const double f0 = sqrt(1.0 - x * x), th = acos(x);
+// An energy with its angle and sqrt(1 - x^2).
+struct Node {
+  double x, th, f0, unused;
+};
+__device__ inline Node node_of(double x) { return Node{x, acos(x), sqrt(1.0 - x * x), 0.0}; }
+__global__ void k_energy_nodes(int grid, int num_div, double xbound, Node *__restrict__ nodes) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_div; i += gridDim.x * blockDim.x)
+    nodes[i] = node_of(grid_energy(grid, i, num_div, xbound));
+}
+
+__device__ inline double2 coef(int kind, const Node &e, int m) {
+  const double f0 = e.f0;
   double sn, cs;
-  sincos(m * th, &sn, &cs);
+  sincos(m * e.th, &sn, &cs);
   if (kind == COEF_DELTA) return make_double2(cs / f0 / M_PI, 0.0);
   const double2 p = make_double2(cs, -sn);  // (x - i f0)^m
   if (kind == COEF_G) return make_double2(p.y / f0, -p.x / f0);  // -i p / f0
-  const double2 q = cmul(p, make_double2(x, m * f0));             // * (x + i m f0)
+  const double2 q = cmul(p, make_double2(e.x, m * f0));           // * (x + i m f0)
   const double inv = 1.0 / (f0 * f0 * f0);
   const double2 dg = make_double2(q.y * inv, -q.x * inv);          // -i q / f0^3
   if (kind == COEF_DG) return dg;
   return make_double2(dg.x + dg.x, 0.0);                           // Re DG + conj(Re DG)
 }
 
-// tab(i, m) = conj(B(x_i, m)): zgemm_cn conjugates its first operand
-__global__ void k_coef_table(int kind, int grid, int num_div, int M1, double xbound, double2 *__restrict__ tab) {
-  const long tot = (long)num_div * M1;
+// Coefficient rows of all energies.  parts 2: B(x_i, m) as (re, im); 1: its real part (the others
+// are real); conjugate: conj(B), for zgemm_cn.  Rows of ld numbers, zero past parts * M1.
+__global__ void k_coef_table(int kind, int num_div, int M1, int ld, int parts, int conjugate,
+                             const Node *__restrict__ nodes, double *__restrict__ tab) {
+  const int per = (ld + parts - 1) / parts;
+  const long tot = (long)num_div * per;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / M1), m = (int)(t % M1);
-    tab[t] = cconj(coef(kind, grid_energy(grid, i, num_div, xbound), m));
+    const int i = (int)(t / per), m = (int)(t % per);
+    double2 c = m < M1 ? coef(kind, nodes[i], m) : make_double2(0.0, 0.0);
+    if (conjugate) c = cconj(c);
+    double *o = tab + (size_t)i * ld + (size_t)m * parts;
+    o[0] = c.x;
+    if (parts == 2) o[1] = c.y;
   }
 }
 
-// kernel_i = pref * sum_m0 (left coefficient x Y), one warp per energy, fixed order
-__global__ void k_energy_sums(int variant, int grid, const double2 *__restrict__ Y1, const double2 *__restrict__ Y2,
-                              int num_div, int M0, double pref, double xbound, double *__restrict__ kern) {
+// Right-hand rows of the real sums: parts 2 (Im of B mu = Br Im mu + Bi Re mu): (Im, Re) of mu;
+// parts 1: Im mu or Re mu.
+__global__ void k_table_rows_real(const double2 *__restrict__ mu, int M0, int M1, int ld, int parts, int imag,
+                                  double *__restrict__ q) {
+  const int per = (ld + parts - 1) / parts;
+  const long tot = (long)M0 * per;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot; t += (long)gridDim.x * blockDim.x) {
+    const int i = (int)(t / per), m = (int)(t % per);
+    const double2 v = m < M1 ? mu[(size_t)i * M1 + m] : make_double2(0.0, 0.0);
+    double *o = q + (size_t)i * ld + (size_t)m * parts;
+    o[0] = imag ? v.y : v.x;
+    if (parts == 2) o[1] = v.x;
+  }
+}
+
+// part[bx][i] = sum over the m0 of column block bx of left(i, m0) Y(i, m0),  Y = P Q^T: P [num_div][ld],
+// Q [M0][ld], real, ld a multiple of 16.  Only one real number per (energy, m0) reaches the
+// output of five of the six sums, so they take one real product (K = 2 M1, or M1 where B is real)
+// in place of a complex one, and Y never leaves the registers: 512 x 512 moments at 15360 energies
+// 0.61 ms (27 of 36 TFLOP/s), where the complex product, its reduction and the sums took 0.94.  FP64 tensor cores (m8n8k4),
+// 128 x 64 outputs per CTA, 8 warps of 32 x 32, K slices of 16 in three cp.async stages (pitch 20:
+// the fragment loads are free of bank conflicts).  left: variant 4 (sea) 2 Im G(m0), else delta(m0).
+constexpr int EBM = 128, EBN = 64, EBK = 16, ELD = EBK + 4, EST = 3;
+
+__device__ __forceinline__ void ecp16(void *smem, const void *g, bool ok) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(g), "r"(ok ? 16 : 0));
+}
+
+__global__ void __launch_bounds__(256, 2)
+    k_energy_gemm(int variant, const double *__restrict__ P, const double *__restrict__ Q, int num_div, int M0, int ld,
+                  const Node *__restrict__ nodes, double *__restrict__ part) {
+  extern __shared__ __align__(16) double esm[];
+  double(*As)[EBM][ELD] = reinterpret_cast<double(*)[EBM][ELD]>(esm);
+  double(*Bs)[EBN][ELD] = reinterpret_cast<double(*)[EBN][ELD]>(esm + EST * EBM * ELD);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = warp >> 1, wn = warp & 1;
+  const int fr = lane >> 2, fk = lane & 3;
+  const int i0 = blockIdx.y * EBM, n0 = blockIdx.x * EBN;
+  const auto load = [&](int st, int k0) {
+#pragma unroll
+    for (int q = 0; q < (EBM + EBN) * EBK / 2 / 256; ++q) {  // 16-byte pieces, 8 a row
+      const int e = threadIdx.x + 256 * q, r = e >> 3, c = (e & 7) * 2;
+      if (r < EBM) {
+        const bool ok = i0 + r < num_div;
+        ecp16(&As[st][r][c], P + (ok ? (size_t)(i0 + r) * ld + k0 + c : 0), ok);
+      } else {
+        const bool ok = n0 + r - EBM < M0;
+        ecp16(&Bs[st][r - EBM][c], Q + (ok ? (size_t)(n0 + r - EBM) * ld + k0 + c : 0), ok);
+      }
+    }
+  };
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nk = ld / EBK;
+#pragma unroll
+  for (int st = 0; st < EST - 1; ++st) {
+    if (st < nk) load(st, st * EBK);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  for (int it = 0; it < nk; ++it) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(EST - 2));
+    __syncthreads();  // slice `it` has landed, and everyone is done with the one before it
+    if (it + EST - 1 < nk) load((it + EST - 1) % EST, (it + EST - 1) * EBK);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const int cur = it % EST;
+#pragma unroll
+    for (int ks = 0; ks < EBK; ks += 4) {
+      double a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = As[cur][wm * 32 + i * 8 + fr][ks + fk];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = Bs[cur][wn * 32 + j * 8 + fr][ks + fk];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                       : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                       : "d"(a[i]), "d"(b[j]));
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __shared__ double rows[2][EBM];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = wm * 32 + i * 8 + fr, e = i0 + r;
+    double sum = 0.0;
+    if (e < num_div) {
+      const Node nd = nodes[e];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m0 = n0 + wn * 32 + j * 8 + 2 * fk + h;
+          if (m0 < M0) {
+            const double c = cos(m0 * nd.th);
+            sum += (variant == 4 ? -2.0 * c / nd.f0 : c / nd.f0 / M_PI) * acc[i][j][h];
+          }
+        }
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (fk == 0) rows[wn][r] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < EBM && i0 + threadIdx.x < num_div)
+    part[(size_t)blockIdx.x * num_div + i0 + threadIdx.x] = rows[0][threadIdx.x] + rows[1][threadIdx.x];
+}
+
+// kern[i] = pref * sum_b part[b][i]  (fixed order)
+__global__ void k_energy_parts(const double *__restrict__ part, int blocks, int num_div, double pref,
+                               double *__restrict__ kern) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < num_div; i += gridDim.x * blockDim.x) {
+    double s = 0.0;
+    for (int b = 0; b < blocks; ++b) s += part[(size_t)b * num_div + i];
+    kern[i] = s * pref;
+  }
+}
+
+// Bastin II: kernel_i = pref * sum_m0 -Re(G(m0) DG(m1) mu - DG(m0) G(m1) mu), one warp per energy,
+// fixed order (Y1 = DG mu, Y2 = G mu, complex)
+__global__ void k_energy_sums2(const double2 *__restrict__ Y1, const double2 *__restrict__ Y2,
+                               const Node *__restrict__ nodes, int num_div, int M0, double pref,
+                               double *__restrict__ kern) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
   if (w >= num_div) return;
-  const double x = grid_energy(grid, w, num_div, xbound);
+  const Node nd = nodes[w];
   double acc = 0.0;
   for (int m0 = l; m0 < M0; m0 += 32) {
-    const double2 y1 = Y1[(size_t)w * M0 + m0];
-    switch (variant) {
-      case 0:  // Bastin: delta(m0) Im(DG(m1) mu)
-      case 1:  // Greenwood: delta(m0) Im(G(m1) mu)
-      case 2:  // Bastin I: as Greenwood
-        acc += coef(COEF_DELTA, x, m0).x * y1.y;
-        break;
-      case 3: {  // Bastin II: -Re(G(m0) DG(m1) mu - DG(m0) G(m1) mu)
-        const double2 y2 = Y2[(size_t)w * M0 + m0];
-        const double2 t = csub(cmul(coef(COEF_G, x, m0), y1), cmul(coef(COEF_DG, x, m0), y2));
-        acc += -t.x;
-        break;
-      }
-      case 4: {  // sea: -Re((G - conj G)(m0) (2 Re DG)(m1) mu)
-        const double2 g = coef(COEF_G, x, m0);
-        acc += -cmul(csub(g, cconj(g)), y1).x;
-        break;
-      }
-      default:  // surface: delta(m0) delta(m1) Re mu
-        acc += coef(COEF_DELTA, x, m0).x * y1.x;
-        break;
-    }
+    const double2 y1 = Y1[(size_t)w * M0 + m0], y2 = Y2[(size_t)w * M0 + m0];
+    const double2 t = csub(cmul(coef(COEF_G, nd, m0), y1), cmul(coef(COEF_DG, nd, m0), y2));
+    acc += -t.x;
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if (l == 0) kern[w] = acc * pref;
@@ -215,11 +338,12 @@ namespace {
 __global__ void k_time_correlation(const double2 *__restrict__ mu, int NT, int T, double x, double scale, double dt,
                                    double *__restrict__ t_out, double *__restrict__ c_out) {
   const double phi = M_PI / (double)(T + 1.0);
+  const Node e = node_of(x);
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < NT; n += gridDim.x * blockDim.x) {
     double out = 0.0;
     for (int m = 0; m < T; ++m) {
       const double g = ((T - m + 1) * cos(phi * m) + sin(phi * m) * cos(phi) / sin(phi)) * phi / M_PI;
-      out += coef(COEF_DELTA, x, m).x * (mu[(size_t)m * NT + n].x * g);
+      out += coef(COEF_DELTA, e, m).x * (mu[(size_t)m * NT + n].x * g);
     }
     t_out[n] = n * dt;
     c_out[n] = out * scale;
@@ -269,26 +393,45 @@ void energy_sums(Session *s, const double2 *mu, int M0, int M1, int N, double ba
                  int variant, int grid, double xbound, int num_div, double *E, double *out) {
   LQ_REQUIRE(variant >= 0 && variant <= 5 && grid >= 0 && grid <= 2 && num_div >= 2, "energy sums: bad argument");
   static const int kind1[6] = {COEF_DG, COEF_G, COEF_G, COEF_DG, COEF_REDG2, COEF_DELTA};
-  double2 *tab = (double2 *)s->get("esum_tab", sizeof(double2) * (size_t)num_div * M1);
-  double2 *Y1 = (double2 *)s->get("esum_y1", sizeof(double2) * (size_t)num_div * M0);
-  double2 *Y2 = variant == 3 ? (double2 *)s->get("esum_y2", sizeof(double2) * (size_t)num_div * M0) : nullptr;
-  double *kern = (double *)s->get("esum_kern", sizeof(double) * (size_t)num_div);
-  const long tot = (long)num_div * M1;
-  const int g = (int)std::max(1L, std::min((tot + 255) / 256, (long)s->sm_count * 16));
-  // Y(i, m0) = sum_m1 conj(tab(i, m1)) mu(m0, m1) = sum_m1 B(x_i, m1) mu(m0, m1)
-  k_coef_table<<<g, 256, 0, s->stream>>>(kind1[variant], grid, num_div, M1, xbound, tab);
-  LQ_LAUNCHED();
-  zgemm_cn(s, tab, num_div, mu, M0, M1, Y1, false);
-  if (Y2) {
-    k_coef_table<<<g, 256, 0, s->stream>>>(COEF_G, grid, num_div, M1, xbound, tab);
-    LQ_LAUNCHED();
-    zgemm_cn(s, tab, num_div, mu, M0, M1, Y2, false);
-  }
   const double a = band_width / 2.0, w = N / a / a;
   const double pref[6] = {-2.0 * w, -w, -w, w / 2 / M_PI, w / 2 / M_PI, M_PI * w};
-  k_energy_sums<<<(num_div * 32 + 255) / 256, 256, 0, s->stream>>>(variant, grid, Y1, Y2, num_div, M0,
-                                                                    pref[variant], xbound, kern);
+  double *kern = (double *)s->get("esum_kern", sizeof(double) * (size_t)num_div);
+  Node *nodes = (Node *)s->get("esum_nodes", sizeof(Node) * (size_t)num_div);
+  k_energy_nodes<<<(num_div + 127) / 128, 128, 0, s->stream>>>(grid, num_div, xbound, nodes);
   LQ_LAUNCHED();
+  const auto blocks_of = [&](long tot) { return (int)std::max(1L, std::min((tot + 255) / 256, (long)s->sm_count * 16)); };
+  if (variant == 3) {
+    double2 *tab = (double2 *)s->get("esum_tab", sizeof(double2) * (size_t)num_div * M1);
+    double2 *Y1 = (double2 *)s->get("esum_y1", sizeof(double2) * (size_t)num_div * M0);
+    double2 *Y2 = (double2 *)s->get("esum_y2", sizeof(double2) * (size_t)num_div * M0);
+    for (double2 *Y : {Y1, Y2}) {
+      // Y(i, m0) = sum_m1 conj(tab(i, m1)) mu(m0, m1) = sum_m1 B(x_i, m1) mu(m0, m1)
+      k_coef_table<<<blocks_of((long)num_div * M1), 256, 0, s->stream>>>(Y == Y1 ? COEF_DG : COEF_G, num_div, M1,
+                                                                         2 * M1, 2, 1, nodes, (double *)tab);
+      LQ_LAUNCHED();
+      zgemm_cn(s, tab, num_div, mu, M0, M1, Y, false);
+    }
+    k_energy_sums2<<<(num_div * 32 + 255) / 256, 256, 0, s->stream>>>(Y1, Y2, nodes, num_div, M0, pref[3], kern);
+    LQ_LAUNCHED();
+  } else {
+    // Im(B mu) for the Bastin and Greenwood kernels; B is real for the sea (Im) and surface (Re) terms
+    const int parts = variant <= 2 ? 2 : 1, ld = (parts * M1 + EBK - 1) / EBK * EBK;
+    double *P = (double *)s->get("esum_tab", sizeof(double) * (size_t)num_div * ld);
+    double *Q = (double *)s->get("esum_q", sizeof(double) * (size_t)M0 * ld);
+    const dim3 g((M0 + EBN - 1) / EBN, (num_div + EBM - 1) / EBM);
+    double *part = (double *)s->get("esum_part", sizeof(double) * (size_t)g.x * num_div);
+    k_coef_table<<<blocks_of((long)num_div * ld / parts), 256, 0, s->stream>>>(kind1[variant], num_div, M1, ld, parts, 0,
+                                                                              nodes, P);
+    LQ_LAUNCHED();
+    k_table_rows_real<<<blocks_of((long)M0 * ld / parts), 256, 0, s->stream>>>(mu, M0, M1, ld, parts, variant != 5, Q);
+    LQ_LAUNCHED();
+    const size_t smem = sizeof(double) * EST * (EBM + EBN) * ELD;
+    raise_smem_limit((const void *)k_energy_gemm, smem);
+    k_energy_gemm<<<g, 256, smem, s->stream>>>(variant, P, Q, num_div, M0, ld, nodes, part);
+    LQ_LAUNCHED();
+    k_energy_parts<<<blocks_of(num_div), 256, 0, s->stream>>>(part, (int)g.x, num_div, pref[variant], kern);
+    LQ_LAUNCHED();
+  }
   k_energy_output<<<1, 1024, 0, s->stream>>>(variant, grid, kern, num_div, xbound, a, band_center, E, out);
   LQ_LAUNCHED();
 }
