@@ -231,7 +231,7 @@ const float2 *DeviceOp::val32() {
     for (long k = 0; k < nnz; ++k) v32[k] = make_float2((float)val[k].x, (float)val[k].y);
     LQ_CUDA(cudaSetDevice(device));
     LQ_CUDA(cudaMalloc(&d_val32, sizeof(float2) * v32.size()));
-    LQ_CUDA(cudaMemcpy(d_val32, v32.data(), sizeof(float2) * v32.size(), cudaMemcpyHostToDevice));
+    to_device(d_val32, v32.data(), sizeof(float2) * v32.size());
   }
   return d_val32;
 }
@@ -253,10 +253,10 @@ void DeviceOp::upload() {
   LQ_CUDA(cudaMalloc(&d_rowptr, sizeof(int) * (n + 1)));
   LQ_CUDA(cudaMalloc(&d_col, sizeof(int) * std::max(1L, nnz)));
   LQ_CUDA(cudaMalloc(&d_val64, sizeof(double2) * std::max(1L, nnz)));
-  LQ_CUDA(cudaMemcpy(d_rowptr, rowptr.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+  to_device(d_rowptr, rowptr.data(), sizeof(int) * (n + 1));
   if (nnz) {
-    LQ_CUDA(cudaMemcpy(d_col, col.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice));
-    LQ_CUDA(cudaMemcpy(d_val64, val.data(), sizeof(double2) * nnz, cudaMemcpyHostToDevice));
+    to_device(d_col, col.data(), sizeof(int) * nnz);
+    to_device(d_val64, val.data(), sizeof(double2) * nnz);
   }
   version++;
 }
@@ -312,10 +312,10 @@ const DeviceOp::Sell &DeviceOp::ensure_sell(int key, bool c64) {
     LQ_CUDA(cudaMalloc(&L.d_off, sizeof(int) * (ns + 1)));
     LQ_CUDA(cudaMalloc(&L.d_col, sizeof(int) * L.len));
     LQ_CUDA(cudaMalloc(&L.d_val64, sizeof(double2) * L.len));
-    LQ_CUDA(cudaMemcpy(L.d_perm, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    LQ_CUDA(cudaMemcpy(L.d_off, off.data(), sizeof(int) * (ns + 1), cudaMemcpyHostToDevice));
-    LQ_CUDA(cudaMemcpy(L.d_col, sc.data(), sizeof(int) * L.len, cudaMemcpyHostToDevice));
-    LQ_CUDA(cudaMemcpy(L.d_val64, sv.data(), sizeof(double2) * L.len, cudaMemcpyHostToDevice));
+    to_device(L.d_perm, order.data(), sizeof(int) * n);
+    to_device(L.d_off, off.data(), sizeof(int) * (ns + 1));
+    to_device(L.d_col, sc.data(), sizeof(int) * L.len);
+    to_device(L.d_val64, sv.data(), sizeof(double2) * L.len);
   }
   if (c64 && !L.d_val32) {
     std::vector<double2> sv(L.len);
@@ -324,7 +324,7 @@ const DeviceOp::Sell &DeviceOp::ensure_sell(int key, bool c64) {
     std::vector<float2> s32(L.len);
     for (size_t q = 0; q < L.len; ++q) s32[q] = make_float2((float)sv[q].x, (float)sv[q].y);
     LQ_CUDA(cudaMalloc(&L.d_val32, sizeof(float2) * L.len));
-    LQ_CUDA(cudaMemcpy(L.d_val32, s32.data(), sizeof(float2) * L.len, cudaMemcpyHostToDevice));
+    to_device(L.d_val32, s32.data(), sizeof(float2) * L.len);
   }
   return L;
 }

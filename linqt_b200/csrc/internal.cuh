@@ -59,6 +59,15 @@ inline int guarded(F &&f) {
     if (!(cond)) ::linqt::fail(LINQT_ERR_INVALID, std::string(msg)); \
   } while (0)
 
+// Host to device on return.  cudaMemcpy alone may return once pageable memory is staged, with the last
+// copy still under way, and the sessions' streams do not wait for the legacy stream it runs on: a
+// kernel launched next could read the previous owner's bytes (a 1.6 MB SELL layout built right
+// before its first recursion was, in about every other run of the tests).
+inline void to_device(void *dst, const void *src, size_t bytes) {
+  LQ_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+  LQ_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // after a launch: surface configuration errors immediately
 #define LQ_LAUNCHED() LQ_CUDA(cudaGetLastError())
 

@@ -219,7 +219,7 @@ void upload(const Plan &pl, int device, DevPlan &d) {
   d.device = device;
   LQ_CUDA(cudaSetDevice(device));
   LQ_CUDA(cudaMalloc(&d.blob, blob.size()));
-  LQ_CUDA(cudaMemcpy(d.blob, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+  to_device(d.blob, blob.data(), blob.size());
   char *b = (char *)d.blob;
   PlanView &v = d.v;
   v.wbb = pl.wbb;
