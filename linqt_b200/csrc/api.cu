@@ -245,6 +245,8 @@ void DeviceOp::upload() {
     val = up_val;
   }
   nnz = rowptr[n];
+  max_row = 0;
+  for (int i = 0; i < n; ++i) max_row = std::max(max_row, rowptr[i + 1] - rowptr[i]);
   free_device();
   loc_order.clear();  // the pattern may have changed (a rescale can add diagonal entries)
   static std::atomic<unsigned long> next_uid{1};

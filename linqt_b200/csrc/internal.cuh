@@ -205,6 +205,7 @@ struct DeviceOp {
   std::vector<int> rowptr, col;
   std::vector<double2> val;
   long nnz = 0;
+  int max_row = 0;  // entries of the longest row
   int *d_rowptr = nullptr, *d_col = nullptr;
   double2 *d_val64 = nullptr;
   unsigned version = 0;  // bumped by rescale
@@ -451,6 +452,7 @@ void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1
 // dots[(r*steps + s)*2 + i] = sums of partials[steps][nb][2] over the nb / nreal CTAs of each realisation
 void reduce_step_partials(Session *s, const double2 *partials, int steps, int nb, int nreal, double2 *dots);
 // the same recursions of small lattices in one cluster (recur_cluster.cu); false: too large
+constexpr int kRegsRow = 16;  // k_recur_1d_regs: entries of the longest row it takes
 bool cluster_recur_1d(Session *s, const DeviceOp &H, const void *phi, const void *x0, int steps, int M, int mode, int R,
                       bool fp32, double2 *dots);
 bool cluster_recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lst, void *Rst, const void *phi, int M,

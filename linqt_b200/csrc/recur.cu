@@ -37,7 +37,6 @@ constexpr int kThreads = 256;
 // L2 latency of a step instead of three (square 256 x 256, one vector: 1449 -> 1272 us for
 // 512 steps).  In k_recur_lr the same costs 2-3 % on blocks beyond L1 (registers) and is not done.
 constexpr int kHoist = 1;
-
 using Barrier = GridBarrier;
 
 // CTAs an SM holds: the gathers are latency-bound, so the registers of more columns per thread
@@ -415,6 +414,78 @@ __global__ void __launch_bounds__(kThreads, min_ctas_1d<T>(VPT))
     if (!grid_wait(bar)) return;
     prev = cur;
     cur = y;
+  }
+}
+
+// The same with one value of the block per thread, for blocks that the co-resident threads cover: what
+// bounds these is the chain of a step (gathers, row sum, store, barrier), not a bandwidth.  So the
+// thread's operator entries and its own T_{s-1}, T_s and phi stay in registers for the whole recursion
+// and all its gathers, at most NR, are in flight at once: one L2 round trip a step, where k_recur_1d
+// reads the entries from shared memory and gathers four at a time.  us a step, k_recur_1d and this:
+// square 256 x 256 2.66, 2.14; honeycomb 97 x 64 of 8 vectors 3.10, 2.35; cubic 24^3 2.93, 2.07;
+// Kane-Mele 48 x 48 of 4 vectors 4.26, 2.17.  The same stores; the dot products' partials are sums
+// over other rows.
+template <class T, int NR, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB)
+    k_recur_1d_regs(int n, int rshift, const int *__restrict__ rp, const int *__restrict__ ci,
+                    const double2 *__restrict__ hv, const typename cplx_t<T>::type *phi,
+                    typename cplx_t<T>::type *x0, typename cplx_t<T>::type *b1, int steps, int M, int mode,
+                    double2 *__restrict__ partials, Barrier *bar) {
+  using C = typename cplx_t<T>::type;
+  grid_init(bar, gridDim.x);
+  const long item = (long)blockIdx.x * kThreads + threadIdx.x;
+  const bool valid = item < ((long)n << rshift);
+  const int row = valid ? (int)(item >> rshift) : 0, col = (int)(item & ((1 << rshift) - 1));
+  const int b = rp[row], cnt = valid ? rp[row + 1] - b : 0;
+  double2 h[NR];
+  unsigned off[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k)
+    if (k < cnt) {
+      h[k] = hv[b + k];
+      off[k] = ((unsigned)ci[b + k] << rshift) + col;
+    }
+  C xc{}, xp{}, f{};
+  if (valid) {
+    xc = x0[item];
+    if (mode == 1) f = phi[item];
+  }
+  for (int s = 0; s < steps; ++s) {
+    const bool need_y = mode == 2 ? (2 * s + 1 < M) : (s + 1 < M);
+    const C *src = s & 1 ? b1 : x0;
+    C x[NR];
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (k < cnt) x[k] = src[off[k]];
+    double2 y = make_double2(0, 0);
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (k < cnt) y = cfma(h[k], x[k], y);
+    if (s) {
+      const double2 p = to_d2(xp);
+      y.x = 2 * y.x - p.x;
+      y.y = 2 * y.y - p.y;
+    }
+    const C yc = from_d2<C>(y);
+    if (need_y && valid) (s & 1 ? x0 : b1)[item] = yc;
+    if (need_y) grid_arrive(bar);
+    double2 d0 = make_double2(0, 0), d1 = d0;
+    const double2 xi = to_d2(xc);
+    if (mode == 1) {
+      d0 = cfma_conj(to_d2(f), xi, d0);
+    } else {
+      d0 = cfma_conj(xi, xi, d0);
+      d1 = cfma_conj(to_d2(yc), xi, d1);
+    }
+    block_sum2(d0, d1);
+    if (threadIdx.x == 0) {
+      partials[((size_t)s * gridDim.x + blockIdx.x) * 2] = d0;
+      partials[((size_t)s * gridDim.x + blockIdx.x) * 2 + 1] = d1;
+    }
+    if (!need_y) break;
+    if (!grid_wait(bar)) return;
+    xp = xc;
+    xc = yc;
   }
 }
 
@@ -883,10 +954,68 @@ void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, vo
   LQ_LAUNCHED();
 }
 
+namespace {
+// False if the threads of a cooperative grid do not cover the block.
+template <class T, int NR, int MINB>
+bool run_1d_regs(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
+                 double2 *dots) {
+  using C = typename cplx_t<T>::type;
+  const void *f = (const void *)k_recur_1d_regs<T, NR, MINB>;
+  const long need = ((long)H.n * R + kThreads - 1) / kThreads;
+  int per_sm = 0;
+  LQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kThreads, 0));
+  if (need > (long)per_sm * s->sm_count) return false;
+  const int grid = coop_grid(s, f, need, 0);
+  if (grid < need) {  // a session with a share of the device
+    coop_share_return(s);
+    return false;
+  }
+  double2 *partials = (double2 *)s->get("rec1d_part", sizeof(double2) * 2 * (size_t)steps * grid);
+  Barrier *bar = barrier_for(s);
+  int n = H.n, rshift = 0;
+  while ((1 << rshift) < R) ++rshift;
+  const C *ph = (const C *)phi;
+  C *xx = (C *)x0, *bb = (C *)b1;
+  void *args[] = {&n,  &rshift, (void *)&H.d_rowptr, (void *)&H.d_col, (void *)&H.d_val64, (void *)&ph, &xx,
+                  &bb, &steps,  &M,                  &mode,            &partials,          &bar};
+  coop_launch(s, f, grid, args, 0);
+  reduce_step_partials(s, partials, steps, grid, 1, dots);
+  return true;
+}
+
+// Rows of up to NR entries.  The fewest CTAs an SM that cover the block leave a thread the most
+// registers: honeycomb 64 x 64 of 4 vectors takes 1.81 us a step with 2, 1.92 with 3 and 2.32 with 4.
+// Wider rows with more CTAs an SM would spill their entries and are left to k_recur_1d.
+template <class T>
+bool recur_1d_regs(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode,
+                   int R, double2 *dots) {
+#define LQ_REGS(NR, MINB) \
+  if (run_1d_regs<T, NR, MINB>(s, H, phi, x0, b1, steps, M, mode, R, dots)) return true
+  if (H.max_row <= 4) {
+    LQ_REGS(4, 2);
+    LQ_REGS(4, 3);
+    LQ_REGS(4, 4);
+  } else if (H.max_row <= 6) {
+    LQ_REGS(6, 2);
+    LQ_REGS(6, 3);
+  } else if (H.max_row <= 8) {
+    LQ_REGS(8, 2);
+  } else if (H.max_row <= kRegsRow) {
+    LQ_REGS(kRegsRow, 1);
+  }
+#undef LQ_REGS
+  return false;
+}
+}  // namespace
+
 void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
               bool fp32, double2 *dots, int sellC, int shape, const void *stacked, int nreal, bool c64,
               bool on_chip) {
   if (on_chip && sellC == 0 && !stacked && !c64 && cluster_recur_1d(s, H, phi, x0, steps, M, mode, R, fp32, dots)) return;
+  if (on_chip && sellC == 0 && !stacked && !c64 &&
+      (fp32 ? recur_1d_regs<float>(s, H, phi, x0, b1, steps, M, mode, R, dots)
+            : recur_1d_regs<double>(s, H, phi, x0, b1, steps, M, mode, R, dots)))
+    return;
   Barrier *bar = barrier_for(s);
   const int Rw = stacked ? R / nreal : R;  // columns per CTA
   if (fp32)

@@ -310,7 +310,9 @@ size_t op_slice_bytes(const DeviceOp &A, int r0, int r1) {
 // honeycomb 8192 x 2 (66k) 3.1 / 3.1, x 4 4.1 / 3.2; Kane-Mele 1024 x 4 (53k) 2.6 / 4.0.  L/R,
 // honeycomb 800 x 16 (141k) 2.9 / 3.6, x 32 4.4 / 3.6; Kane-Mele 4096 x 1 (135k) 3.1 / 7.6,
 // honeycomb 8192 x 1 (90k) 2.8 / 3.4, x 2 3.8 / 3.5.
-constexpr long kClGathers1d = 80000, kClGathersLr = 140000;
+// k_recur_1d_regs, rows of up to kRegsRow entries, is a faster grid kernel: square 12100 x 1 (60k)
+// 1.70 / 1.91, 14400 x 1 (72k) 2.03 / 1.93; cubic 8000 x 1 (56k) 1.86 / 2.15, 10648 x 1 (75k) 2.26 / 2.15.
+constexpr long kClGathers1d = 80000, kClGathersRegs = 65000, kClGathersLr = 140000;
 
 ClGeom cluster_geometry(Session *s, const void *func, const DeviceOp &H, const DeviceOp *V, int R, size_t esz,
                         int blocks) {
@@ -318,7 +320,8 @@ ClGeom cluster_geometry(Session *s, const void *func, const DeviceOp &H, const D
   // tests of the bounded grid barrier need the grid kernels
   if (s->inject_extra || s->inject_limit) return g;
   const long items = (long)H.n * R;
-  if (blocks == 4 ? (2 * H.nnz + (V ? V->nnz : 0)) * R > kClGathersLr : H.nnz * R > kClGathers1d) return g;
+  const long line = blocks == 4 ? kClGathersLr : blocks == 2 && H.max_row <= kRegsRow ? kClGathersRegs : kClGathers1d;
+  if ((blocks == 4 ? 2 * H.nnz + (V ? V->nnz : 0) : H.nnz) * R > line) return g;
   const size_t limit = 227 * 1024;
   while ((1 << g.rshift) < R) ++g.rshift;
   const int want = (int)std::min<long>(kClMax, std::max<long>(1, (items + kClItems - 1) / kClItems));
