@@ -124,6 +124,48 @@ __device__ __forceinline__ void gather_fma(double2 h, const C *p, double2 (&acc)
   for (int u = 0; u < V; ++u) acc[u] = cfma(h, t[u], acc[u]);
 }
 
+// B entries k, k + st, ... of a row times their columns of x (TWO: and of x2): all gathers first.
+template <int B, bool TWO, class HV, class C, int V>
+__device__ __forceinline__ void gather_batch(const int *ci, const HV *hv, int k, int st, int ldx, const C *x,
+                                             double2 (&acc)[V], const C *x2, double2 (&acc2)[V]) {
+  C t[B][V], t2[TWO ? B : 1][V];
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const size_t off = (size_t)ci[k + i * st] * ldx;
+    ld_row<V>(x + off, t[i]);
+    if constexpr (TWO) ld_row<V>(x2 + off, t2[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const double2 h = to_d2(hv[k + i * st]);
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      acc[u] = cfma(h, t[i][u], acc[u]);
+      if constexpr (TWO) acc2[u] = cfma(h, t2[i][u], acc2[u]);
+    }
+  }
+}
+
+// acc = a row (entries b, b + st, ... below e) times x, TWO: acc2 times x2; x and x2 point at this
+// thread's columns.  The kernels are bound by these dependent round trips.  Four entries go at a time, and
+// the one to three that are left at once too; the compiler's loop over the rest takes them one by one,
+// half of the round trips of a row of 7.  ms a solve with that loop and this: cubic 100^3, 64 vectors
+// (rows of 7) 52.9, 49.5; 4 cubic 40^3 FP32 6.68, 6.44; Kane-Mele 64 x 64, 32 vectors (rows of 13 and 7)
+// 56.3, 54.4, in mixed precision 15.7, 14.6; honeycomb 48 x 40, 3 vectors (4 and 3) 1.41, 1.33.
+template <bool TWO, class HV, class C, int V>
+__device__ __forceinline__ void gather_row(const int *ci, const HV *hv, int b, int e, int st, int ldx, const C *x,
+                                           double2 (&acc)[V], const C *x2, double2 (&acc2)[V]) {
+  int k = b;
+#pragma unroll 1
+  for (; e - k > 3 * st; k += 4 * st) gather_batch<4, TWO>(ci, hv, k, st, ldx, x, acc, x2, acc2);
+  if (e - k > 2 * st)
+    gather_batch<3, TWO>(ci, hv, k, st, ldx, x, acc, x2, acc2);
+  else if (e - k > st)
+    gather_batch<2, TWO>(ci, hv, k, st, ldx, x, acc, x2, acc2);
+  else if (e - k > 0)
+    gather_batch<1, TWO>(ci, hv, k, st, ldx, x, acc, x2, acc2);
+}
+
 __device__ __forceinline__ double2 shfl_down2(double2 v, int o) {
   v.x = __shfl_down_sync(0xffffffffu, v.x, o);
   v.y = __shfl_down_sync(0xffffffffu, v.y, o);
@@ -256,21 +298,16 @@ __global__ void __launch_bounds__(kThreads, min_ctas_lr(VPT))
       // the previous vectors of this row, read after the gathers
       if (doL && pL) prefetch_l2(pL + base);
       if (yR && pR) prefetch_l2(pR + base);
-#pragma unroll 4
-      for (int k = b; k < e; k += st) {
-        const int j = ci[k];
-        const double2 h = hv[k];
-        const size_t off = (size_t)j * R + c0;
-        if (doL) gather_fma<C, VPT>(h, xL + off, aL);
-        gather_fma<C, VPT>(h, xR + off, aR);
-      }
+      if (doL)
+        gather_row<true>(ci, hv, b, e, st, R, xL + c0, aL, xR + c0, aR);
+      else
+        gather_row<false>(ci, hv, b, e, st, R, xR + c0, aR, (const C *)nullptr, aL);
       if (HAS_V) {
         double2 aV[VPT];
 #pragma unroll
         for (int u = 0; u < VPT; ++u) aV[u] = make_double2(0, 0);
         const int vb = vrp[row], ve = vrp[row + 1];
-#pragma unroll 4
-        for (int k = vb; k < ve; ++k) gather_fma<C, VPT>(vv[k], xR + (size_t)vci[k] * R + c0, aV);
+        gather_row<false>(vci, vv, vb, ve, 1, R, xR + c0, aV, (const C *)nullptr, aL);
         C o[VPT];
 #pragma unroll
         for (int u = 0; u < VPT; ++u) o[u] = from_d2<C>(aV[u]);
@@ -372,8 +409,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_1d<T>(VPT))
       } else {
         if (prev) prefetch_l2(prev + base);
       }
-#pragma unroll 4
-      for (int k = b; k < e; k += st) gather_fma<C, VPT>(to_d2(hv[k]), cur + (size_t)ci[k] * ldx + coff + c0, acc);
+      gather_row<false>(ci, hv, b, e, st, ldx, cur + coff + c0, acc, (const C *)nullptr, acc);
       C yv[VPT];
       if constexpr (VPT > kHoist) {
         if (prev) ld_row<VPT>(prev + base, pv);
@@ -537,8 +573,7 @@ __global__ void __launch_bounds__(kThreads, VPT <= 2 ? 4 : VPT == 4 ? 3 : 2)
         for (int u = 0; u < VPT; ++u) xv[u] = X[base + u];
       }
       const int kb = rp[pos], ke = rp[pos + 1];
-#pragma unroll 4
-      for (int k = kb; k < ke; ++k) gather_fma<double2, VPT>(hv[k], cur + (size_t)ci[k] * RW + c0, acc);
+      gather_row<false>(ci, hv, kb, ke, 1, RW, (const double2 *)cur + c0, acc, (const double2 *)nullptr, acc);
       if constexpr (VPT > kHoist) {
         if (prev) ld_row<VPT>(prev + base, pv);
 #pragma unroll
