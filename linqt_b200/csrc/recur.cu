@@ -33,9 +33,11 @@ namespace linqt {
 namespace {
 
 constexpr int kThreads = 256;
-// Columns per thread up to which the 1D kernels load a row's own vectors before its gathers: one
-// L2 latency of a step instead of three (square 256 x 256, one vector: 1449 -> 1272 us for
-// 512 steps).  In k_recur_lr the same costs 2-3 % on blocks beyond L1 (registers) and is not done.
+// Columns per thread up to which a row's own vectors are loaded before its gathers: one L2 latency of a
+// step instead of three (square 256 x 256, one vector: 1449 -> 1272 us for 512 steps).  k_recur_lr, us a
+// step after the gathers and before: Kane-Mele 16384 x 32 FP64 20.8, 19.6, 65536 x 32 81.4, 80.2;
+// honeycomb 32768 x 8 7.25, 6.75, 32768 x 32 23.4, 20.9, 8192 x 16 5.06, 4.74.  With four FP32 columns
+// the registers weigh as much (Kane-Mele 16384 x 16 9.72, 9.85; honeycomb 32768 x 32 15.75, 15.20).
 constexpr int kHoist = 1;
 using Barrier = GridBarrier;
 
@@ -295,9 +297,15 @@ __global__ void __launch_bounds__(kThreads, min_ctas_lr(VPT))
 #pragma unroll
       for (int u = 0; u < VPT; ++u) aL[u] = aR[u] = make_double2(0, 0);
       const size_t base = (size_t)row * R + c0;
-      // the previous vectors of this row, read after the gathers
-      if (doL && pL) prefetch_l2(pL + base);
-      if (yR && pR) prefetch_l2(pR + base);
+      // the previous vectors of this row: kHoist, or read after the gathers
+      C qL[VPT], qR[VPT];
+      if constexpr (VPT <= kHoist) {
+        if (doL && pL) ld_row<VPT>(pL + base, qL);
+        if (yR && pR) ld_row<VPT>(pR + base, qR);
+      } else {
+        if (doL && pL) prefetch_l2(pL + base);
+        if (yR && pR) prefetch_l2(pR + base);
+      }
       if (doL)
         gather_row<true>(ci, hv, b, e, st, R, xL + c0, aL, xR + c0, aR);
       else
@@ -316,11 +324,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas_lr(VPT))
       if (doL) {
         C o[VPT];
         if (pL) {
-          C p[VPT];
-          ld_row<VPT>(pL + base, p);
+          if constexpr (VPT > kHoist) ld_row<VPT>(pL + base, qL);
 #pragma unroll
           for (int u = 0; u < VPT; ++u) {
-            const double2 q = to_d2(p[u]);
+            const double2 q = to_d2(qL[u]);
             o[u] = from_d2<C>(make_double2(2 * aL[u].x - q.x, 2 * aL[u].y - q.y));
           }
         } else {
@@ -332,11 +339,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas_lr(VPT))
       if (yR) {
         C o[VPT];
         if (pR) {
-          C p[VPT];
-          ld_row<VPT>(pR + base, p);
+          if constexpr (VPT > kHoist) ld_row<VPT>(pR + base, qR);
 #pragma unroll
           for (int u = 0; u < VPT; ++u) {
-            const double2 q = to_d2(p[u]);
+            const double2 q = to_d2(qR[u]);
             o[u] = from_d2<C>(make_double2(2 * aR[u].x - q.x, 2 * aR[u].y - q.y));
           }
         } else {
