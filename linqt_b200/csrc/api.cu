@@ -702,7 +702,7 @@ static void realisations_stacked(Session *s, const DeviceOp *const *Hs, int S, c
     PhaseScope ph(s, PH_RECURSION);
     chunk_block(s, states, N, R, 0, R, phi, fp32);
     LQ_CUDA(cudaMemcpyAsync(b0, phi, blk, cudaMemcpyDeviceToDevice, s->stream));
-    recur_1d(s, H0, phi, b0, b1, steps, M, 2, R, fp32, dots, 0, recur_default_shape((long)N * R, Rs, fp32, false), vals, S,
+    recur_1d(s, H0, phi, b0, b1, steps, M, 2, R, fp32, dots, 0, recur_stacked_shape((long)N * R, Rs, fp32), vals, S,
              c64);
     ph.launches(3);
   }

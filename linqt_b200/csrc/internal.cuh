@@ -437,6 +437,7 @@ void moments1d_from_dots_stream(cudaStream_t st, const double2 *dots, int steps,
 int recur_shapes(int R);
 // the shapes the recursions use when nothing else chooses one (items = values of a block)
 int recur_default_shape(long items, int R, bool fp32, bool locality);
+int recur_stacked_shape(long items, int Rs, bool fp32);
 int recur_lr_default_shape(long items, int R, bool fp32);
 void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, void *Rstore, const void *phi,
               void *tbuf, int M, int R, bool fp32, int sellC, int shape = 0);

@@ -976,6 +976,16 @@ int recur_default_shape(long items, int R, bool fp32, bool locality) {
   return shape_with(R, fp32 && items > 400000 ? 4 : 2);
 }
 
+// Stacked realisations of Rs columns each, `items` values in all: a row's columns lie S Rs apart, and one
+// launch holds S times the threads, so more columns a thread pay later than in one block.  us a step
+// with 1, 2 and 4 columns, cubic L^3, S x Rs: FP64 24: 4 x 8 (442k) 9.5, 10.5; 40: 2 x 8 (1.0M) 16.6,
+// 15.1, 4 x 8 37.2, 28.9, 4 x 4 (1.0M) 20.4, 24.4; 64: 4 x 8 145, 113, 4 x 4 84, 86, 3 x 2 (1.6M) 40, 51.
+// FP32 24: 4 x 8 8.1, 10.2, 13.4, 4 x 4 (221k) 7.8, 10.2; 40: 4 x 8 26.5, 21.9, 25.9, 2 x 4 (512k) 9.5,
+// 8.7, 10.0, 3 x 2 9.1, 11.4; 64: 4 x 8 135, 91, 92, 4 x 4 76, 71, 95, 3 x 2 32, 36.
+int recur_stacked_shape(long items, int Rs, bool fp32) {
+  return items > 480000 && Rs >= (fp32 ? 4 : 8) ? shape_with(Rs, 2) : 0;
+}
+
 // The L/R kernel holds twice the sums: FP64 blocks keep shape 0 (Kane-Mele 16384 x 32: 22.2 us with
 // one column, 25.7 with two); large FP32 ones take four columns (Kane-Mele 65536 x 32: 81.6, 88.8
 // and 75.2; honeycomb 131072 x 32: 95.2, 106.0 and 85.3; 8192 x 32: 7.5, 8.1 and 6.6).
