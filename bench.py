@@ -540,19 +540,20 @@ def main():
                 "frac": ach / hbm_peak, "peak_source": peak_src}
     else:
         ach = phases[dom]["flops"] / (phases[dom]["ms"] * 1e-3) / 1e12
-        roof = {"kernel": {"contraction": "zgemm_cn_f64 (mu_nm contraction)", "fft": "kubo_fft (per-site DFTs)"}[dom],
+        roof = {"kernel": {"contraction": "mu_nm contraction", "fft": "kubo_fft (per-site DFTs)"}[dom],
                 "bound": "tensor", "pipe": "fp64", "achieved": ach, "peak": fp64_peak, "unit": "TFLOP/s",
                 "frac": ach / fp64_peak, "peak_source": "FP64 DGEMM (torch.matmul 8192^3) measured in this run"}
         if dom == "contraction" and prec == lq.PREC_FP64:
-            # the kernel forms each complex product with 3 real products (Gauss) instead of the
-            # 4 the algorithmic count assumes: the DMMA work it executes is 3/4 of it
-            roof["executed_frac"] = 0.75 * ach / fp64_peak
-            roof["executed_note"] = "3-product complex form: executed DMMA flops = 3/4 of the algorithmic 8*M^2*K"
-    # DRAM bytes per launch of the dominant kernel: ncu capture of the 64x64-cell case
+            # the complex FP64 product runs as 34 exact INT8 products (17 moduli, two real products each);
+            # the phase also holds the residues and the Chinese remainders
+            ops = 34 * 2.0 * M * M * K / (phases[dom]["ms"] * 1e-3) / 1e12
+            roof.update(kernel="k_residues, k_rns_gemm, k_rns_crt (mu_nm contraction)", pipe="int8", achieved=ops,
+                        peak=2 * bf16_peak, unit="TOP/s", frac=ops / (2 * bf16_peak),
+                        peak_source="twice the measured bf16 GEMM rate", algorithmic_fp64_tflops=ach)
+    # DRAM bytes per launch of the per-site transforms: ncu capture of the 64x64-cell case
     # (M = 256, K = 65,536; dram__bytes_read.sum + dram__bytes_write.sum), scaled by M*K,
-    # which the operand reads of both kernels are proportional to
-    traffic_per_mk = {"contraction": (566779904 + 27903744) / (256 * 65536),
-                      "fft": (545405952 + 114432) / (256 * 65536)}
+    # which their operand reads are proportional to
+    traffic_per_mk = {"fft": (545405952 + 114432) / (256 * 65536)}
     roof["traffic"] = (traffic_per_mk[dom] * M * K) if dom in traffic_per_mk else None
     roof["traffic_unit"] = "bytes per launch (scaled from the 64x64-cell ncu capture)"
     rec_ach = phases["recursion"]["bytes"] / (phases["recursion"]["ms"] * 1e-3) / 1e9
