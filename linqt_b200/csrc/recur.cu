@@ -117,15 +117,6 @@ __device__ __forceinline__ void st_row(float2 *p, const float2 (&v)[V]) {
   }
 }
 
-// acc[u] += h * x[u]
-template <class C, int V>
-__device__ __forceinline__ void gather_fma(double2 h, const C *p, double2 (&acc)[V]) {
-  C t[V];
-  ld_row<V>(p, t);
-#pragma unroll
-  for (int u = 0; u < V; ++u) acc[u] = cfma(h, t[u], acc[u]);
-}
-
 // B entries k, k + st, ... of a row times their columns of x (TWO: and of x2): all gathers first.
 template <int B, bool TWO, class HV, class C, int V>
 __device__ __forceinline__ void gather_batch(const int *ci, const HV *hv, int k, int st, int ldx, const C *x,
