@@ -927,8 +927,8 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
   char *Ls = (char *)s->get("lr_L", blk * M);
   char *Rs = (char *)s->get("lr_R", blk * M);
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
-  double2 *raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * (size_t)M * M);  // hi, lo
-  LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * (size_t)M * M, s->stream));
+  double2 *raw = (double2 *)s->get("mu_raw", sizeof(double2) * (size_t)M * M);
+  LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * (size_t)M * M, s->stream));
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
     {
@@ -938,7 +938,7 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
     }
     {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + (size_t)M * M);
+      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw);
       ph.launches(2);
     }
   }
@@ -994,13 +994,14 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   double2 *raw = nullptr, *acc = nullptr, *acc_c = nullptr, *tab = nullptr;
   const size_t MM = (size_t)M * M;
   if (mu) {
-    raw = (double2 *)s->get("mu_raw", sizeof(double2) * 2 * MM);  // hi, lo
-    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * 2 * MM, s->stream));
+    raw = (double2 *)s->get("mu_raw", sizeof(double2) * MM);
+    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * MM, s->stream));
   }
   // sigma's site sums: from the raw table in double-double (kubo_table.cu), once per solve, or from
   // the transforms of every site (kubo_fft.cu), by the times both take at these sizes; the FP64
   // moments need the same table, so there only what the residues cost beyond the FP64 kernel
-  // (0.9 ps per value of K and 64 x 64 tile) counts
+  // (0.9 ps per value of K and 64 x 64 tile) counts.  A chunk whose table is rejected goes to the
+  // transforms after all, on the device: the two parts of sigma's sums add up.
   size_t planes = 0;
   if (out) {
     const long K = (long)N * ch.Rc;
@@ -1010,11 +1011,9 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     if (kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
       planes = rns_plane_bytes(s, M, M, K);
     acc = (double2 *)s->get("kubo_acc", sizeof(double2) * 2 * (size_t)nump);
+    LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
     if (!planes) {
-      LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
       acc_c = (double2 *)s->get("kubo_acc_c", sizeof(double2) * 2 * (size_t)nump);
-    } else if (mu && !fp32) {
-      tab = raw;
     } else {
       tab = (double2 *)s->get("kubo_tab", sizeof(double2) * 2 * MM);
       LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
@@ -1027,21 +1026,26 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
       chunk_block(s, states, N, R, c * ch.Rc, ch.Rc, phi, fp32);
       ph.launches(1 + lr_vectors(s, H, opl, opr, phi, M, ch.Rc, fp32, Ls, Rs, tmp, o.format, o.step_launches != 0));
     }
+    const long K = (long)N * ch.Rc;
+    const int *rejected = nullptr;
     if (mu) {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, raw + MM, fp32 ? 0 : planes);
+      if (tab && !fp32)
+        rejected = mu_contract_rns(s, Ls, Rs, M, K, false, planes, raw, tab);
+      else
+        mu_contract(s, Ls, Rs, M, K, fp32, o.precision, raw);
       ph.launches(2);
     }
-    if (out && !(tab && tab == raw)) {
+    if (out) {
       PhaseScope ph(s, PH_FFT);
       if (tab) {
-        zgemm_cn_rns(s, Ls, M, Rs, M, (long)N * ch.Rc, fp32, planes, tab, tab + MM);
-        ph.launches(3);
+        if (!rejected) rejected = mu_contract_rns(s, Ls, Rs, M, K, fp32, planes, nullptr, tab);
+        kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc, rejected);
       } else {
-        kubo_fft_sites(s, Ls, Rs, (long)N * ch.Rc, M, nump, formula, fp32, acc_c);
+        kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc_c);
         add_into(s, acc, acc_c, 2 * nump);
-        ph.launches(4);
       }
+      ph.launches(4);
     }
   }
   if (tab) {

@@ -342,20 +342,31 @@ void moments1d_from_dots(Session *s, const double2 *dots, int steps, int M, int 
 // mu_raw[M x M] += sum_k conj(L[m0][k]) * Rv[m1][k], FP64 (or FP32-input) operands
 // C(i,j) (+)= sum_k conj(A[i][k]) B[j][k], FP64
 void zgemm_cn(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, double2 *C, bool accumulate);
-// raw_lo takes the low parts of a contraction that gives more than FP64 (mu_rns.cu); with
-// planes > 0 an FP64 contraction goes there whatever its shape
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw, double2 *raw_lo, size_t planes = 0);
-// Contraction in residues on the INT8 tensor cores, exact up to the 53-bit rounding of its inputs
-// (mu_rns.cu).  rns_faster: whether an FP64 product is faster there; rns_us: its time;
+                 double2 *mu_raw);
+// The same from the residues (mu_rns.cu), and the table in double-double into tab [2][M][M] (hi, lo);
+// mu_raw (FP64 blocks) or tab may be NULL.  Returns the device's judgement: where it is 1, the residues'
+// rounding could have moved the table, mu_raw got the FP64 kernel's sum and tab nothing.
+const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, size_t planes,
+                           double2 *mu_raw, double2 *tab);
+// Contraction in residues on the INT8 tensor cores, exact up to the rounding of its inputs
+// to a common exponent (mu_rns.cu).  rns_faster: whether an FP64 product is faster there; rns_us: its time;
 // rns_bytes: the planes of the whole product; rns_plane_bytes: the planes it gets (0: memory is
 // short, use the FP64 kernel).
 bool rns_faster(int MA, int MB, long K);
 double rns_us(int M, long K);
 size_t rns_bytes(int MA, int MB, long K);
 size_t rns_plane_bytes(Session *s, int MA, int MB, long K);
-void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
-                  size_t plane_bytes, double2 *raw_hi, double2 *raw_lo);
+struct RnsStats;
+struct RnsSide;
+struct RnsJudgement {
+  RnsStats *stats;
+  RnsSide *side;
+  int nchunk;
+};
+RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
+                          size_t plane_bytes, double2 *sum_hi, double2 *sum_lo);
+void rns_clear_stats(Session *s);
 void mu_finalize(Session *s, const double2 *mu_raw, int M, int R, double2 *mu);
 void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 *dst);
 // R random-phase states (R x N, state-major) from Philox4x32-10 with the given seed (states.cu)
@@ -387,9 +398,10 @@ inline size_t i8_digit_bytes(int digits, int M, long K) {
 // FFT path: accumulate p/w over all sites into acc[2*nump] (complex)
 // prefactors pf_m of Kubo_solver_FFT (kubo_fft.cu)
 void kubo_prefactors(Session *s, int M, int nump, double2 *pf);
+// only_if: acc += them, on the device where *only_if is set
 void kubo_fft_sites(Session *s, const void *L, const void *Rv, long nsites, int M, int nump, int formula,
-                    bool fp32_inputs, double2 *acc);
-// the same from the raw moment table hi + lo (kubo_table.cu); its time, and that of the site
+                    bool fp32_inputs, double2 *acc, const int *only_if = nullptr);
+// acc += the same from the raw moment table hi + lo (kubo_table.cu); its time, and that of the site
 // transforms of one call (us)
 void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc);
 double kubo_table_us(int M, int nump, int formula);

@@ -13,8 +13,9 @@
 // and ket_m = R_m[l] (= OPR T_m(H) phi).  Products of the transforms are summed over
 // sites into p[k] (and w[k]).
 //
-// These kernels serve solves with few sites, or few sites per energy; larger ones take the sums from
-// the moment table (kubo_table.cu), by the times of kubo_sites_us and kubo_table_us.
+// These kernels serve solves with few sites, or few sites per energy, and blocks whose table was
+// rejected (mu_rns.cu); other large ones take the sums from the moment table (kubo_table.cu), by
+// the times of kubo_sites_us and kubo_table_us.
 //
 // Design: one CTA per site at a time (persistent, the CTAs interleaved over the sites),
 // all 8 (or 4) transforms of the site in shared memory.  nump = 16 * 16 * R3,
@@ -232,7 +233,8 @@ __device__ __forceinline__ void greenwood_product_reg(const double2 (&x)[4], dou
 template <int R3, int NSEQ, bool HALF, class Tin>
 __global__ void __launch_bounds__(kFftThreads)
     k_kubo_fft(const Tin *__restrict__ L, const Tin *__restrict__ Rv, long K, long chunk, int M,
-               const double2 *__restrict__ pf_g, double2 *__restrict__ part) {
+               const double2 *__restrict__ pf_g, double2 *__restrict__ part, const int *only_if) {
+  if (only_if && !*only_if) return;
   constexpr int P = 16 * R3;     // n / 16
   constexpr int n = 16 * P;      // nump
   constexpr int ROW = P + 1;     // padded row of the 16 x P arrangement
@@ -380,8 +382,10 @@ __global__ void __launch_bounds__(kFftThreads)
 template <int NSEQ, class Tin>
 __global__ void __launch_bounds__(256)
     k_kubo_dft(const Tin *__restrict__ L, const Tin *__restrict__ Rv, long K, long chunk, int M, int nump,
-               const double2 *__restrict__ pf_g, const double2 *__restrict__ twg, double2 *__restrict__ part) {
+               const double2 *__restrict__ pf_g, const double2 *__restrict__ twg, double2 *__restrict__ part,
+               const int *only_if) {
   extern __shared__ double2 sm[];
+  if (only_if && !*only_if) return;
   double2 *bk = sm;  // bra[M], ket[M]
   const int kpt = (nump + blockDim.x - 1) / blockDim.x;
   double2 *acc_g = part + (size_t)blockIdx.x * 2 * nump;
@@ -435,9 +439,10 @@ __global__ void k_twiddles(int n, double2 *__restrict__ tw) {
 }
 
 // acc[t] = sum_b part[b][t]: 32 outputs a CTA, 8 threads each striding over b, then in order (one
-// thread per output: 107 us for 592 CTAs' partials)
+// thread per output: 107 us for 592 CTAs' partials).  only_if: acc += it where *only_if is set.
 __global__ void __launch_bounds__(256)
-    k_sum_parts(const double2 *__restrict__ part, int nb, int len, double2 *__restrict__ acc) {
+    k_sum_parts(const double2 *__restrict__ part, int nb, int len, double2 *__restrict__ acc, const int *only_if) {
+  if (only_if && !*only_if) return;
   __shared__ double2 sh[8][32];
   const int l = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int t = blockIdx.x * 32 + l;
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (g == 0 && t < len) {
     for (int q = 1; q < 8; ++q) s = cadd(s, sh[q][l]);
-    acc[t] = s;
+    acc[t] = only_if ? cadd(acc[t], s) : s;
   }
 }
 
@@ -496,7 +501,8 @@ __global__ void k_kubo_post(const double2 *__restrict__ acc, double R, int nump,
 }
 
 template <int R3, int NSEQ, class Tin>
-void launch_fft(Session *s, const Tin *L, const Tin *Rv, long K, int M, const double2 *pf, double2 *acc) {
+void launch_fft(Session *s, const Tin *L, const Tin *Rv, long K, int M, const double2 *pf, double2 *acc,
+                const int *only_if) {
   constexpr int n = 256 * R3;
   const size_t smem = sizeof(double2) * ((size_t)NSEQ * 16 * (16 * R3 + 1) + 16 * 16 * R3 + 16 * R3 + (size_t)M) +
                       sizeof(Tin) * 4 * (size_t)M;
@@ -511,21 +517,22 @@ void launch_fft(Session *s, const Tin *L, const Tin *Rv, long K, int M, const do
   // halves cover the R3 outputs), so the partials need no clearing
   if (2 * M <= n) {
     raise_smem_limit((const void *)k_kubo_fft<R3, NSEQ, true, Tin>, smem);
-    k_kubo_fft<R3, NSEQ, true, Tin><<<nb, kFftThreads, smem, s->stream>>>(L, Rv, K, chunk, M, pf, part);
+    k_kubo_fft<R3, NSEQ, true, Tin><<<nb, kFftThreads, smem, s->stream>>>(L, Rv, K, chunk, M, pf, part, only_if);
   } else {
     raise_smem_limit((const void *)k_kubo_fft<R3, NSEQ, false, Tin>, smem);
-    k_kubo_fft<R3, NSEQ, false, Tin><<<nb, kFftThreads, smem, s->stream>>>(L, Rv, K, chunk, M, pf, part);
+    k_kubo_fft<R3, NSEQ, false, Tin><<<nb, kFftThreads, smem, s->stream>>>(L, Rv, K, chunk, M, pf, part, only_if);
   }
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) coop_share_return(s);
   LQ_CUDA(le);
   coop_share_hand_back(s);
-  k_sum_parts<<<(2 * n + 31) / 32, 256, 0, s->stream>>>(part, nb, 2 * n, acc);
+  k_sum_parts<<<(2 * n + 31) / 32, 256, 0, s->stream>>>(part, nb, 2 * n, acc, only_if);
   LQ_LAUNCHED();
 }
 
 template <int NSEQ, class Tin>
-void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump, const double2 *pf, double2 *acc) {
+void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump, const double2 *pf, double2 *acc,
+                const int *only_if) {
   double2 *tw = (double2 *)s->get("kubo_tw", sizeof(double2) * nump);
   k_twiddles<<<(nump + 255) / 256, 256, 0, s->stream>>>(nump, tw);
   LQ_LAUNCHED();
@@ -535,9 +542,9 @@ void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump
   const int nb = (int)std::max(1L, std::min(K, (long)s->sm_count * 4));
   const long chunk = (K + nb - 1) / nb;
   double2 *part = (double2 *)s->get("kubo_part", sizeof(double2) * 2 * (size_t)nump * nb);
-  k_kubo_dft<NSEQ, Tin><<<nb, 256, smem, s->stream>>>(L, Rv, K, chunk, M, nump, pf, tw, part);
+  k_kubo_dft<NSEQ, Tin><<<nb, 256, smem, s->stream>>>(L, Rv, K, chunk, M, nump, pf, tw, part, only_if);
   LQ_LAUNCHED();
-  k_sum_parts<<<(2 * nump + 31) / 32, 256, 0, s->stream>>>(part, nb, 2 * nump, acc);
+  k_sum_parts<<<(2 * nump + 31) / 32, 256, 0, s->stream>>>(part, nb, 2 * nump, acc, only_if);
   LQ_LAUNCHED();
 }
 
@@ -548,20 +555,23 @@ bool shared_memory_fft(int nump, int formula) {
 
 template <class Tin>
 void kubo_fft_sites_t(Session *s, const Tin *L, const Tin *Rv, long nsites, int M, int nump, int formula,
-                      const double2 *pf, double2 *acc) {
+                      const double2 *pf, double2 *acc, const int *oi) {
   const bool bastin = formula == LINQT_KUBO_BASTIN;
+#define LQ_FFT(r3) \
+  bastin ? launch_fft<r3, 8>(s, L, Rv, nsites, M, pf, acc, oi) : launch_fft<r3, 4>(s, L, Rv, nsites, M, pf, acc, oi)
   if (shared_memory_fft(nump, formula)) {
     switch (nump) {
-      case 256: bastin ? launch_fft<1, 8>(s, L, Rv, nsites, M, pf, acc) : launch_fft<1, 4>(s, L, Rv, nsites, M, pf, acc); return;
-      case 512: bastin ? launch_fft<2, 8>(s, L, Rv, nsites, M, pf, acc) : launch_fft<2, 4>(s, L, Rv, nsites, M, pf, acc); return;
-      case 1024: bastin ? launch_fft<4, 8>(s, L, Rv, nsites, M, pf, acc) : launch_fft<4, 4>(s, L, Rv, nsites, M, pf, acc); return;
-      case 2048: launch_fft<8, 4>(s, L, Rv, nsites, M, pf, acc); return;
+      case 256: LQ_FFT(1); return;
+      case 512: LQ_FFT(2); return;
+      case 1024: LQ_FFT(4); return;
+      case 2048: launch_fft<8, 4>(s, L, Rv, nsites, M, pf, acc, oi); return;
     }
   }
+#undef LQ_FFT
   if (bastin)
-    launch_dft<8>(s, L, Rv, nsites, M, nump, pf, acc);
+    launch_dft<8>(s, L, Rv, nsites, M, nump, pf, acc, oi);
   else
-    launch_dft<4>(s, L, Rv, nsites, M, nump, pf, acc);
+    launch_dft<4>(s, L, Rv, nsites, M, nump, pf, acc, oi);
 }
 
 }  // namespace
@@ -582,13 +592,13 @@ void kubo_prefactors(Session *s, int M, int nump, double2 *pf) {
 }
 
 void kubo_fft_sites(Session *s, const void *Lv, const void *Rvv, long nsites, int M, int nump, int formula,
-                    bool fp32_inputs, double2 *acc) {
+                    bool fp32_inputs, double2 *acc, const int *only_if) {
   double2 *pf = (double2 *)s->get("kubo_pf", sizeof(double2) * M);
   kubo_prefactors(s, M, nump, pf);
   if (fp32_inputs)
-    kubo_fft_sites_t(s, (const float2 *)Lv, (const float2 *)Rvv, nsites, M, nump, formula, pf, acc);
+    kubo_fft_sites_t(s, (const float2 *)Lv, (const float2 *)Rvv, nsites, M, nump, formula, pf, acc, only_if);
   else
-    kubo_fft_sites_t(s, (const double2 *)Lv, (const double2 *)Rvv, nsites, M, nump, formula, pf, acc);
+    kubo_fft_sites_t(s, (const double2 *)Lv, (const double2 *)Rvv, nsites, M, nump, formula, pf, acc, only_if);
 }
 
 void kubo_postprocess(Session *s, const double2 *acc, int R, int nump, int formula, int N, double band_width,

@@ -201,8 +201,8 @@ __global__ void k_table_sum(const double2 *__restrict__ part, int groups, int n,
     dd_acc(make_double2(__shfl_down_sync(0xffffffffu, w.x, o), __shfl_down_sync(0xffffffffu, w.y, o)), w);
   }
   if (lane == 0) {
-    acc[k] = make_double2(p.x + p.y, 0.0);
-    acc[n + k] = make_double2(0.0, w.x + w.y);
+    acc[k].x += p.x + p.y;
+    acc[n + k].y += w.x + w.y;
   }
 }
 
@@ -232,8 +232,8 @@ double kubo_table_us(int M, int nump, int formula) {
   return 40 + work * (formula == LINQT_KUBO_BASTIN ? 1.0 : 0.5) / 8.8e6;
 }
 
-// acc (as kubo_fft_sites gives it, with the parts of p and w that reach sigma) from the raw
-// table hi + lo [M][M].
+// acc += what kubo_fft_sites gives (the parts of p and w that reach sigma), from the raw table
+// hi + lo [M][M].
 void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc) {
   const int n = nump, A = best_split(M, n), P = 2 * n / A;
   const int IB = std::max(1, std::min(P, kTabPairs / A));

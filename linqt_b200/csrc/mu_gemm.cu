@@ -13,7 +13,9 @@
 // on 64x64 complex output tiles per CTA (8 warps of 32x16), cp.async double-buffered
 // 16-deep K slices in padded shared memory (conflict-free fragment loads), split-K over
 // the long K axis with a fixed-order FP64 reduction (deterministic).
+#include "dd.cuh"
 #include "internal.cuh"
+#include "rns_judge.cuh"
 
 namespace linqt {
 
@@ -76,8 +78,8 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 // conj(A) B = (t1 - t2) + i (t3 - t1 - t2) in the epilogue -- 3/4 of the tensor-core work of
 // the four-product form, at the cost of one rounding-level cancellation in the imaginary part.
 template <class Tc>
-__global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ L, const Tc *__restrict__ Rv, int MA,
-                                                         int MB, long K, long kchunk, double2 *__restrict__ part) {
+__device__ __forceinline__ void zgemm_block(const Tc *__restrict__ L, const Tc *__restrict__ Rv, int MA, int MB, long K,
+                                            long kchunk, double2 *__restrict__ part) {
   extern __shared__ double2 smem_d[];
   Tc *smem = reinterpret_cast<Tc *>(smem_d);
   Tc(*As)[BM][LDS] = reinterpret_cast<Tc(*)[BM][LDS]>(smem);
@@ -160,6 +162,74 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
   }
 }
 
+template <class Tc>
+__global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ L, const Tc *__restrict__ Rv, int MA,
+                                                         int MB, long K, long kchunk, double2 *__restrict__ part) {
+  zgemm_block(L, Rv, MA, MB, K, kchunk, part);
+}
+
+// Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo.  Where it is
+// rejected, raw += the FP64 product, by the grid of k_zgemm_cn_f64 (the last CTA of a tile adds its
+// parts, in order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that
+// the usual one costs 5 us and no host decision.
+__global__ void __launch_bounds__(256, 2)
+    k_commit(RnsStats *stats, RnsSide *side, int nchunk, const double2 *__restrict__ hi,
+             const double2 *__restrict__ lo, const double2 *__restrict__ L, const double2 *__restrict__ Rv, int M, long K,
+             long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
+             double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo) {
+  __shared__ bool last;
+  const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)));
+  const int m0 = blockIdx.y * BM, m1 = blockIdx.x * BN;
+  if (!no) {
+    for (int e = threadIdx.x + 256 * blockIdx.z; e < BM * BN; e += 256 * gridDim.z) {
+      const int i = m0 + e / BN, j = m1 + e % BN;
+      if (i >= M || j >= M) continue;
+      const size_t t = (size_t)i * M + j;
+      const double2 h = hi[t];
+      if (raw) raw[t] = cadd(raw[t], h);
+      if (tab_hi) {
+        const double2 l = lo[t], th = tab_hi[t], tl = tab_lo[t];
+        const double2 re = dd_add(make_double2(th.x, tl.x), make_double2(h.x, l.x));
+        const double2 im = dd_add(make_double2(th.y, tl.y), make_double2(h.y, l.y));
+        tab_hi[t] = make_double2(re.x, im.x);
+        tab_lo[t] = make_double2(re.y, im.y);
+      }
+    }
+  } else if (raw) {
+    zgemm_block(L, Rv, M, M, K, kchunk, part);
+    unsigned *count = tiles + blockIdx.y * gridDim.x + blockIdx.x;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.z - 1;
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      for (int e = threadIdx.x; e < BM * BN; e += 256) {
+        const int i = m0 + e / BN, j = m1 + e % BN;
+        if (i >= M || j >= M) continue;
+        const size_t t = (size_t)i * M + j;
+        double2 s = raw[t];
+        for (unsigned z = 0; z < gridDim.z; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
+        raw[t] = s;
+      }
+      if (threadIdx.x == 0) *count = 0;
+    }
+  }
+  // every CTA has judged before the last one clears the statistics
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd(&stats->done, 1u) == gridDim.x * gridDim.y * gridDim.z - 1;
+  __syncthreads();
+  if (!last) return;
+  const int words = 2 * nchunk * (int)(sizeof(RnsSide) / sizeof(unsigned long long));
+  for (int t = threadIdx.x; t < words; t += 256) reinterpret_cast<unsigned long long *>(side)[t] = 0;
+  if (threadIdx.x == 0) {
+    stats->top = 0;
+    stats->done = 0;
+    stats->rejected = no;
+  }
+}
+
 // mu_raw += sum_z part[z]  (fixed order over z)
 __global__ void k_reduce_parts(const double2 *__restrict__ part, int S, long MM, double2 *__restrict__ mu_raw) {
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < MM; t += (long)gridDim.x * blockDim.x) {
@@ -210,8 +280,11 @@ __global__ void k_moments1d(const double2 *__restrict__ dots, int steps, int M, 
   }
 }
 
-template <class Tc>
-void zgemm_cn_t(Session *s, const Tc *A, int MA, const Tc *B, int MB, long K, double2 *C, bool accumulate) {
+// The split of K of the FP64 kernel: S slices of kchunk.
+struct KSplit {
+  long S, kchunk;
+};
+KSplit split_k(Session *s, int MA, int MB, long K) {
   const int tiles = ((MA + BM - 1) / BM) * ((MB + BN - 1) / BN);
   const long target = (long)s->sm_count * 2 * 2;
   long S = std::max(1L, (target + tiles - 1) / tiles);
@@ -219,17 +292,22 @@ void zgemm_cn_t(Session *s, const Tc *A, int MA, const Tc *B, int MB, long K, do
   S = std::max(1L, std::min(std::min(S, 64L), (K + min_chunk - 1) / min_chunk));
   long kchunk = (K + S - 1) / S;
   kchunk = (kchunk + BK - 1) / BK * BK;
-  S = (K + kchunk - 1) / kchunk;
-  double2 *part = (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)S * MA * MB);
-  const size_t smem = sizeof(Tc) * 2 * (BM + BN) * LDS;
-  raise_smem_limit((const void *)k_zgemm_cn_f64<Tc>, smem);
-  dim3 grid((MB + BN - 1) / BN, (MA + BM - 1) / BM, (unsigned)S);
-  k_zgemm_cn_f64<Tc><<<grid, 256, smem, s->stream>>>(A, B, MA, MB, K, kchunk, part);
+  return {(K + kchunk - 1) / kchunk, kchunk};
+}
+constexpr size_t zgemm_smem(size_t esz) { return esz * 2 * (BM + BN) * LDS; }
+
+template <class Tc>
+void zgemm_cn_t(Session *s, const Tc *A, int MA, const Tc *B, int MB, long K, double2 *C, bool accumulate) {
+  const KSplit k = split_k(s, MA, MB, K);
+  double2 *part = (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MA * MB);
+  raise_smem_limit((const void *)k_zgemm_cn_f64<Tc>, zgemm_smem(sizeof(Tc)));
+  dim3 grid((MB + BN - 1) / BN, (MA + BM - 1) / BM, (unsigned)k.S);
+  k_zgemm_cn_f64<Tc><<<grid, 256, zgemm_smem(sizeof(Tc)), s->stream>>>(A, B, MA, MB, K, k.kchunk, part);
   LQ_LAUNCHED();
   const long MM = (long)MA * MB;
   if (!accumulate) LQ_CUDA(cudaMemsetAsync(C, 0, sizeof(double2) * MM, s->stream));
   const int g2 = (int)std::max(1L, std::min((MM + 255) / 256, (long)s->sm_count * 8));
-  k_reduce_parts<<<g2, 256, 0, s->stream>>>(part, (int)S, MM, C);
+  k_reduce_parts<<<g2, 256, 0, s->stream>>>(part, (int)k.S, MM, C);
   LQ_LAUNCHED();
 }
 
@@ -247,12 +325,31 @@ void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 
   LQ_LAUNCHED();
 }
 
+const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, size_t planes,
+                           double2 *mu_raw, double2 *tab) {
+  LQ_REQUIRE(!(fp32_inputs && mu_raw), "residues: moments of FP64 blocks only");
+  const size_t MM = (size_t)M * M;
+  const KSplit k = mu_raw ? split_k(s, M, M, K) : KSplit{1, K};
+  const dim3 grid((M + BN - 1) / BN, (M + BM - 1) / BM, (unsigned)k.S);
+  double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MM) : nullptr;
+  unsigned *tiles = (unsigned *)s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
+  double2 *sum = (double2 *)s->get("rns_sum", sizeof(double2) * 2 * MM);
+  const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, planes, sum, sum + MM);
+  const size_t smem = zgemm_smem(sizeof(double2));
+  raise_smem_limit((const void *)k_commit, smem);
+  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, sum, sum + MM, (const double2 *)L,
+                                           (const double2 *)Rv, M, K, k.kchunk, part, tiles, mu_raw, tab,
+                                           tab ? tab + MM : nullptr);
+  LQ_LAUNCHED();
+  return &j.stats->rejected;
+}
+
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw, double2 *raw_lo, size_t planes) {
+                 double2 *mu_raw) {
   if (!fp32_inputs) {
-    if (!planes && rns_faster(M, M, K)) planes = rns_plane_bytes(s, M, M, K);
+    const size_t planes = rns_faster(M, M, K) ? rns_plane_bytes(s, M, M, K) : 0;
     if (planes)
-      zgemm_cn_rns(s, L, M, Rv, M, K, false, planes, mu_raw, raw_lo);
+      (void)mu_contract_rns(s, L, Rv, M, K, false, planes, mu_raw, nullptr);
     else
       zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
   } else if (i8_digits(precision)) {

@@ -18,11 +18,20 @@
 //     (k_rns_gemm, tcgen05 kind::i8), each reduced mod p in its epilogue.
 //  4. The Chinese remainder theorem gives the exact integer sums (|Re|, |Im| <= 2^107 K,
 //     below half the product of the moduli), scaled back and added over the chunks in
-//     double-double arithmetic (k_rns_crt).
+//     double-double arithmetic (k_rns_crt).  The sum comes as hi + lo, so that the energy
+//     reconstruction (kubo_table.cu) may use more than 53 bits of it.
+//  5. The sum is accepted or not, on the device (judge in rns_judge.cuh, k_commit in mu_gemm.cu).
 //
-// Against the FP64 tensor-core kernel (mu_gemm.cu), whose partial sums round once per term,
-// the only error is that of step 1, which averages over K.  raw comes as hi + lo, so that the
-// energy reconstruction (kubo_fft.cu) may use more than 53 bits of it.
+// Against the FP64 tensor-core kernel (mu_gemm.cu), whose partial sums round once per term, the
+// only error is that of step 1, which averages over K: a value keeps the bits above 2^-53 of its
+// row chunk's largest, not 53 of its own.  Where the sides are large on the same sites, that is
+// no loss (a disordered chain, currents everywhere: random states 1.1e-17 of the table's maximum, a
+// local state 1.4e-16; FP64 products 1.6e-16 and 3.5e-16).  Where one is large only where the other
+// is small, the table lives on the small values: currents in two regions that the states hardly
+// connect were off by 5e-11 of the maximum, or all of it (FP64 products 5e-16).  So step 1's error
+// is estimated from what it did, the rows' units and norms (rns_judge.cuh), and a sum that it could
+// move by more than kAccept of the maximum is dropped for the FP64 kernel's, and sigma's for
+// the site transforms.  That costs one launch, 5 us, and 0.2 % of the contraction of 1024 moments.
 //
 // Measured (contraction phase, before = the FP64 kernel): Kane-Mele 64 x 64 cells, M = 1024,
 // K = 524288: 121.0 -> 30.5 ms; graphene 128 x 128, M = 512, K = 262144: 15.2 -> 5.8 ms.  The
@@ -37,6 +46,7 @@
 
 #include "dd.cuh"
 #include "internal.cuh"
+#include "rns_judge.cuh"
 #include "tc_common.cuh"
 
 namespace linqt {
@@ -116,6 +126,7 @@ constexpr int kBk = 128;             // K bytes of a GEMM block (one swizzle row
 constexpr int kChunkMax = 32768;
 constexpr int kPart = 4096;          // K (complex) that a CTA of k_residues holds in registers
 constexpr int kBadExp = 1 << 20;     // exponent mark of a chunk with a non-finite value
+static_assert(kChunkMax <= kMaxParts * kPart, "parts of a chunk");
 
 // ---------------------------------------------------------------------------
 // residues
@@ -143,9 +154,10 @@ template <class Tc>
 __global__ void __launch_bounds__(256, 2)
     k_residues(const Tc *__restrict__ srcA, const Tc *__restrict__ srcB, long ld, long K, int kc, int rows_a,
                int rows_b, int nkb, int8_t *__restrict__ plA, int8_t *__restrict__ plB, int *__restrict__ expA,
-               int *__restrict__ expB, int nchunk) {
+               int *__restrict__ expB, int nchunk, RnsSide *__restrict__ side) {
   __shared__ unsigned red[8];
   __shared__ unsigned part_max;
+  __shared__ double part_sq[8];
   cg::cluster_group cl = cg::this_cluster();
   const bool b_side = blockIdx.z & 1;
   const int c = blockIdx.z >> 1, row = blockIdx.y;
@@ -189,6 +201,7 @@ __global__ void __launch_bounds__(256, 2)
   const size_t plane = (size_t)nkb * rows * kBk;
   int8_t *out = (b_side ? plB : plA) + (size_t)c * kPlanes * plane + (size_t)row * kBk + lane * 4;
   constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52
+  double sq = 0.0;  // sum of squares, in units of 2^(2 (e - 53))
 #pragma unroll 1
   for (int g = 0; g < 4; ++g) {
     const int kb = (base >> 7) + g * 8 + warp;
@@ -204,6 +217,7 @@ __global__ void __launch_bounds__(256, 2)
       xi[q] = (double)ib;
       lr[q] = (int)ia;
       li[q] = (int)ib;
+      sq = fma(xr[q], xr[q], fma(xi[q], xi[q], sq));
     }
 #pragma unroll
     for (int h = 0; h < 3; ++h)  // rotate: v[0] is the next group
@@ -227,6 +241,17 @@ __global__ void __launch_bounds__(256, 2)
       *reinterpret_cast<uint32_t *>(o + (size_t)(2 * j) * plane) = low_bytes(u[0], u[1], u[2], u[3]);
       *reinterpret_cast<uint32_t *>(o + (size_t)(2 * j + 1) * plane) = low_bytes(w[0], w[1], w[2], w[3]);
     }
+  }
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  if (lane == 0) part_sq[warp] = sq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += part_sq[w];
+    RnsSide &sd = side[blockIdx.z];
+    const double unit = bad ? INFINITY : __hiloint2double((1023 - 53 + e) << 20, 0);
+    if (blockIdx.x == 0) raise_to(&sd.unit, unit);
+    raise_to(&sd.sq[blockIdx.x], bad ? INFINITY : t * unit * unit);
   }
 }
 
@@ -481,17 +506,24 @@ __device__ __forceinline__ double2 dd_from_i128(__int128 X, int ex) {
   return make_double2(ldexp(v.x, ex), ldexp(v.y, ex));
 }
 
-// raw(i, j) += sum over chunks of 2^(ea + eb - 106) X, X the integer with the residues of the
-// planes; one thread per entry, chunks in order, all in double-double.
+// sum(i, j) (+)= sum over chunks of 2^(ea + eb - 106) X, X the integer with the residues of the
+// planes; one thread per entry, chunks in order, all in double-double.  The last slab of chunks
+// also leaves the sum's largest value.
 __global__ void __launch_bounds__(256)
     k_rns_crt(const uint8_t *__restrict__ res, int pitch, int MA, int MB, int nchunk, const int *__restrict__ expA,
-              const int *__restrict__ expB, double2 *__restrict__ raw_hi, double2 *__restrict__ raw_lo) {
+              const int *__restrict__ expB, bool first, bool last, RnsStats *__restrict__ stats,
+              double2 *__restrict__ sum_hi, double2 *__restrict__ sum_lo) {
   const u128 P = ((u128)kProdHi << 64) | kProdLo;
   const size_t plane = (size_t)MA * pitch;
+  unsigned long long top = 0;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < (long)MA * MB; t += (long)gridDim.x * blockDim.x) {
     const int i = (int)(t / MB), j = (int)(t % MB);
-    const double2 hi = raw_hi[t], lo = raw_lo[t];
-    double2 re = make_double2(hi.x, lo.x), im = make_double2(hi.y, lo.y);
+    double2 re = make_double2(0.0, 0.0), im = re;
+    if (!first) {
+      const double2 hi = sum_hi[t], lo = sum_lo[t];
+      re = make_double2(hi.x, lo.x);
+      im = make_double2(hi.y, lo.y);
+    }
     for (int c = 0; c < nchunk; ++c) {
       const int ea = expA[(size_t)i * nchunk + c], eb = expB[(size_t)j * nchunk + c];
       if (ea == kBadExp || eb == kBadExp) {
@@ -520,9 +552,14 @@ __global__ void __launch_bounds__(256)
       re = dd_add(re, dd_from_i128(xr, ea + eb - 106));
       im = dd_add(im, dd_from_i128(xi, ea + eb - 106));
     }
-    raw_hi[t] = make_double2(re.x, im.x);
-    raw_lo[t] = make_double2(re.y, im.y);
+    sum_hi[t] = make_double2(re.x, im.x);
+    sum_lo[t] = make_double2(re.y, im.y);
+    top = max(top, max((unsigned long long)__double_as_longlong(fabs(re.x)),
+                       (unsigned long long)__double_as_longlong(fabs(im.x))));
   }
+  if (!last) return;
+  for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(&stats->top, top);
 }
 
 // [blocks][rows][128 bytes], box 128 bytes x 128 rows; rows past the end read as zero
@@ -588,10 +625,10 @@ size_t rns_plane_bytes(Session *s, int MA, int MB, long K) {
   return 0;
 }
 
-// raw (hi + lo, MA x MB) += sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K),
-// with planes of at most plane_bytes bytes at a time.
-void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
-                  size_t plane_bytes, double2 *raw_hi, double2 *raw_lo) {
+// sum (hi + lo, MA x MB) = sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K),
+// with planes of at most plane_bytes bytes at a time, and what it is to be judged by.
+RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
+                          size_t plane_bytes, double2 *sum_hi, double2 *sum_lo) {
   // K chunks of equal length, a multiple of the GEMM block, short enough for one set of planes
   const size_t per_k = (size_t)kPlanes * (MA + MB);
   long cap = std::min<long>(kChunkMax, (long)(plane_bytes / per_k) / kBk * kBk);
@@ -607,6 +644,9 @@ void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long
   uint8_t *res = (uint8_t *)s->get("rns_res", (size_t)slab * kPlanes * MA * pitch);
   int *eA = (int *)s->get("rns_exp", sizeof(int) * (size_t)(MA + MB) * slab);
   int *eB = eA + (size_t)MA * slab;
+  // "counter": zeroed when they are allocated
+  RnsStats *stats = (RnsStats *)s->get("mu_judge_counter", sizeof(RnsStats));
+  RnsSide *side = (RnsSide *)s->get("mu_sides_counter", sizeof(RnsSide) * 2 * (size_t)nchunk_all);
   int *err = (int *)s->get("mu_tc_err_barrier", sizeof(int) * 4);  // read by mu_tc_check_error
   s->barrier_used = true;
   const CUtensorMap ta = make_map_rns(plA, MA, (long)nkb * kPlanes * slab),
@@ -629,17 +669,27 @@ void zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long
     cfg.numAttrs = 1;
     if (fp32_inputs)
       LQ_CUDA(cudaLaunchKernelEx(&cfg, k_residues<float2>, (const float2 *)A + k0, (const float2 *)B + k0, K, len, kc,
-                                 MA, MB, nkb, plA, plB, eA, eB, nc));
+                                 MA, MB, nkb, plA, plB, eA, eB, nc, side + 2 * c0));
     else
       LQ_CUDA(cudaLaunchKernelEx(&cfg, k_residues<double2>, (const double2 *)A + k0, (const double2 *)B + k0, K, len,
-                                 kc, MA, MB, nkb, plA, plB, eA, eB, nc));
+                                 kc, MA, MB, nkb, plA, plB, eA, eB, nc, side + 2 * c0));
     const long tiles = (long)((MA + kRnsTile - 1) / kRnsTile) * ((MB + kRnsTile - 1) / kRnsTile) * kPlanes * nc;
     const int pairs = (int)std::max(1L, std::min(tiles, (long)s->sm_count / 2));
     k_rns_gemm<<<2 * pairs, kRnsThreads, smem, s->stream>>>(ta, tb, MA, MB, len, kc, nkb, nc, res, pitch, err);
     LQ_LAUNCHED();
     const int g = (int)std::max(1L, std::min(((long)MA * MB + 255) / 256, (long)s->sm_count * 8));
-    k_rns_crt<<<g, 256, 0, s->stream>>>(res, pitch, MA, MB, nc, eA, eB, raw_hi, raw_lo);
+    k_rns_crt<<<g, 256, 0, s->stream>>>(res, pitch, MA, MB, nc, eA, eB, c0 == 0, c0 + nc == nchunk_all,
+                                        stats, sum_hi, sum_lo);
     LQ_LAUNCHED();
+  }
+  return {stats, side, (int)nchunk_all};
+}
+
+// After a wait that expired: the statistics of the contractions so far are void.
+void rns_clear_stats(Session *s) {
+  for (const char *name : {"mu_judge_counter", "mu_sides_counter", "mu_tiles_counter"}) {
+    auto it = s->ws.find(name);
+    if (it != s->ws.end()) LQ_CUDA(cudaMemsetAsync(it->second.first, 0, it->second.second, s->stream));
   }
 }
 

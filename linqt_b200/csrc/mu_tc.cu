@@ -271,7 +271,10 @@ int mu_tc_check_error(Session *s) {
   int h = 0;
   LQ_CUDA(cudaMemcpyAsync(&h, it->second.first, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   LQ_CUDA(cudaStreamSynchronize(s->stream));
-  if (h) LQ_CUDA(cudaMemsetAsync(it->second.first, 0, sizeof(int), s->stream));
+  if (h) {
+    LQ_CUDA(cudaMemsetAsync(it->second.first, 0, sizeof(int), s->stream));
+    rns_clear_stats(s);
+  }
   return h;
 }
 
