@@ -54,7 +54,7 @@ void *Session::get(const std::string &name, size_t bytes) {
   }
   void *p = nullptr;
   cudaError_t e = cudaMallocAsync(&p, bytes, stream);
-  if (e == cudaErrorMemoryAllocation) {
+  const auto retry = [&] {
     // Blocks freed earlier stay cached in the pool, each in its own address range, so a
     // larger buffer may not fit although the bytes are there: once this stream has reached
     // its frees, hand the pool's unused memory back and try once more.
@@ -63,7 +63,10 @@ void *Session::get(const std::string &name, size_t bytes) {
     if (cudaStreamSynchronize(stream) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess)
       cudaMemPoolTrimTo(pool, 0);
     e = cudaMallocAsync(&p, bytes, stream);
-  }
+  };
+  if (e == cudaErrorMemoryAllocation) retry();
+  // the residue planes are an option (mu_rns.cu): they give way to any other buffer
+  if (e == cudaErrorMemoryAllocation && name.rfind("rns_", 0) != 0 && release("rns_")) retry();
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(LINQT_ERR_NOMEM, "cudaMallocAsync(" + std::to_string(bytes) + ") for '" + name + "' failed: " +
@@ -84,6 +87,21 @@ void Session::drop_graphs() {
   for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
   graphs.clear();
   graph_calls.clear();
+}
+
+bool Session::release(const char *prefix) {
+  bool any = false;
+  for (auto it = ws.begin(); it != ws.end();) {
+    if (it->first.rfind(prefix, 0) == 0) {
+      if (!any) drop_graphs();
+      any = true;
+      cudaFreeAsync(it->second.first, stream);
+      it = ws.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  return any;
 }
 
 void Session::trim() {
@@ -344,6 +362,15 @@ static size_t free_device_bytes() {
   size_t fr = 0, tot = 0;
   LQ_CUDA(cudaMemGetInfo(&fr, &tot));
   return fr;
+}
+
+size_t free_pool_bytes(int device) {
+  cudaMemPool_t pool = nullptr;
+  uint64_t reserved = 0, used = 0;
+  LQ_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
+  LQ_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  LQ_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return free_device_bytes() + (size_t)(reserved > used ? reserved - used : 0);
 }
 
 // states (R x N, device) -> chunk c of width Rc (power of two) as an N x Rc block
@@ -1001,23 +1028,20 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   // the transforms of every site (kubo_fft.cu), by the times both take at these sizes; the FP64
   // moments need the same table, so there only what the residues cost beyond the FP64 kernel
   // (0.9 ps per value of K and 64 x 64 tile) counts.  A chunk whose table is rejected goes to the
-  // transforms after all, on the device: the two parts of sigma's sums add up.
-  size_t planes = 0;
+  // transforms after all, on the device, and a chunk whose planes do not fit here: the two parts of
+  // sigma's sums add up.
   if (out) {
     const long K = (long)N * ch.Rc;
     const double tiles = (M + 63) / 64, f64_us = 75 + 9.0e-4 * tiles * tiles * K;
     double extra_us = rns_us(M, K);
     if (mu && !fp32) extra_us = rns_faster(M, M, K) ? 0 : std::max(0.0, extra_us - f64_us);
-    if (kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
-      planes = rns_plane_bytes(s, M, M, K);
     acc = (double2 *)s->get("kubo_acc", sizeof(double2) * 2 * (size_t)nump);
+    acc_c = (double2 *)s->get("kubo_acc_c", sizeof(double2) * 2 * (size_t)nump);
     LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
-    if (!planes) {
-      acc_c = (double2 *)s->get("kubo_acc_c", sizeof(double2) * 2 * (size_t)nump);
-    } else {
-      tab = (double2 *)s->get("kubo_tab", sizeof(double2) * 2 * MM);
-      LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
-    }
+    if (s->rns_budget &&
+        kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
+      tab = kubo_table_reserve(s, M, nump);
+    if (tab) LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
   }
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
@@ -1028,18 +1052,21 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     }
     const long K = (long)N * ch.Rc;
     const int *rejected = nullptr;
+    int slab = 0;
     if (mu) {
       PhaseScope ph(s, PH_CONTRACT);
-      if (tab && !fp32)
-        rejected = mu_contract_rns(s, Ls, Rs, M, K, false, planes, raw, tab);
+      if (tab && !fp32) slab = mu_reserve_rns(s, M, K, true);
+      if (slab)
+        rejected = mu_contract_rns(s, Ls, Rs, M, K, false, slab, raw, tab);
       else
         mu_contract(s, Ls, Rs, M, K, fp32, o.precision, raw);
       ph.launches(2);
     }
     if (out) {
       PhaseScope ph(s, PH_FFT);
-      if (tab) {
-        if (!rejected) rejected = mu_contract_rns(s, Ls, Rs, M, K, fp32, planes, nullptr, tab);
+      if (tab && !(mu && !fp32)) slab = mu_reserve_rns(s, M, K, false);
+      if (slab) {
+        if (!rejected) rejected = mu_contract_rns(s, Ls, Rs, M, K, fp32, slab, nullptr, tab);
         kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc, rejected);
       } else {
         kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc_c);

@@ -272,7 +272,8 @@ struct Session {
   long phase_launches[4] = {0, 0, 0, 0};
   int sm_count = 148;
   size_t hbm_budget = 0;  // chunking budget; 0 = what the device has free
-  size_t rns_budget = 8ull << 30;  // residue planes of the FP64 contraction (mu_rns.cu), at most
+  size_t rns_budget = 8ull << 30;  // residue planes of the FP64 contraction (mu_rns.cu); 0: none
+  bool strict_memory = false;      // an optional buffer that does not fit fails the solve (served beside others)
   bool barrier_used = false;  // a persistent kernel ran since the last error check
   // fault injection for tests (linqt_session_inject_barrier_timeout): grid barriers await
   // inject_extra more CTAs than launched and give up after inject_limit polls
@@ -295,11 +296,13 @@ struct Session {
   void drop_graphs();
 
   void *get(const std::string &name, size_t bytes);  // cached device buffer, >= bytes
+  bool release(const char *prefix);  // gives back the workspaces whose names begin so; whether any
   void trim();
   ~Session();
 };
 
 Session *default_session();
+size_t free_pool_bytes(int device);  // free on the device or cached in its pool
 Session *resolve(linqt_session *s);
 
 // scoped phase timer (CUDA events on the session stream when timing is on)
@@ -346,26 +349,28 @@ void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool 
                  double2 *mu_raw);
 // The same from the residues (mu_rns.cu), and the table in double-double into tab [2][M][M] (hi, lo);
 // mu_raw (FP64 blocks) or tab may be NULL.  Returns the device's judgement: where it is 1, the residues'
-// rounding could have moved the table, mu_raw got the FP64 kernel's sum and tab nothing.
-const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, size_t planes,
+// rounding could have moved the table, mu_raw got the FP64 kernel's sum and tab nothing.  `slab` is
+// what mu_reserve_rns gave just before: not 0.
+int mu_reserve_rns(Session *s, int M, long K, bool moments);
+const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int slab,
                            double2 *mu_raw, double2 *tab);
 // Contraction in residues on the INT8 tensor cores, exact up to the rounding of its inputs
 // to a common exponent (mu_rns.cu).  rns_faster: whether an FP64 product is faster there; rns_us: its time;
-// rns_bytes: the planes of the whole product; rns_plane_bytes: the planes it gets (0: memory is
-// short, use the FP64 kernel).
+// rns_reserve: the chunks of K at a time whose buffers it holds (0: memory is short, use the FP64
+// kernel); rns_footprint: their bytes.
 bool rns_faster(int MA, int MB, long K);
 double rns_us(int M, long K);
-size_t rns_bytes(int MA, int MB, long K);
-size_t rns_plane_bytes(Session *s, int MA, int MB, long K);
+int rns_reserve(Session *s, int MA, int MB, long K);
+size_t rns_footprint(int MA, int MB, long K, size_t budget);
 struct RnsStats;
 struct RnsSide;
 struct RnsJudgement {
+  const double2 *hi, *lo;  // the sum
   RnsStats *stats;
   RnsSide *side;
   int nchunk;
 };
-RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
-                          size_t plane_bytes, double2 *sum_hi, double2 *sum_lo);
+RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab);
 void rns_clear_stats(Session *s);
 void mu_finalize(Session *s, const double2 *mu_raw, int M, int R, double2 *mu);
 void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 *dst);
@@ -403,6 +408,8 @@ void kubo_fft_sites(Session *s, const void *L, const void *Rv, long nsites, int 
                     bool fp32_inputs, double2 *acc, const int *only_if = nullptr);
 // acc += the same from the raw moment table hi + lo (kubo_table.cu); its time, and that of the site
 // transforms of one call (us)
+// (kubo_table_reserve: whether its buffers are held, the table [2][M][M] among them)
+double2 *kubo_table_reserve(Session *s, int M, int nump);
 void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc);
 double kubo_table_us(int M, int nump, int formula);
 double kubo_sites_us(long nsites, int M, int nump, int formula);

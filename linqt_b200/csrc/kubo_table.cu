@@ -232,17 +232,56 @@ double kubo_table_us(int M, int nump, int formula) {
   return 40 + work * (formula == LINQT_KUBO_BASTIN ? 1.0 : 0.5) / 8.8e6;
 }
 
+namespace {
+struct TableGrid {
+  int A, P, IB, blocks, groups;
+};
+TableGrid table_grid(const Session *s, int M, int n) {
+  TableGrid g;
+  g.A = best_split(M, n);
+  g.P = 2 * n / g.A;
+  g.IB = std::max(1, std::min(g.P, kTabPairs / g.A));
+  g.blocks = (g.P + g.IB - 1) / g.IB;
+  g.groups = std::max(1, std::min(M, 4 * s->sm_count / g.blocks));
+  return g;
+}
+struct TableBuffers {
+  double2 *cosines, *coef, *part, *table;
+  double *amp;
+};
+TableBuffers table_buffers(Session *s, int M, int n) {
+  const size_t MM = (size_t)M * M;
+  TableBuffers b;
+  b.cosines = (double2 *)s->get("kt_cos", sizeof(double2) * 4 * (size_t)n);
+  b.amp = (double *)s->get("kt_amp", sizeof(double) * (size_t)M);
+  b.coef = (double2 *)s->get("kt_coef", sizeof(double2) * 2 * MM);
+  b.part = (double2 *)s->get("kt_part", sizeof(double2) * 2 * (size_t)table_grid(s, M, n).groups * (n + 1));
+  b.table = (double2 *)s->get("kt_table", sizeof(double2) * 2 * MM);
+  return b;
+}
+}  // namespace
+
+// The raw table's buffer, with all that kubo_table_sums needs beside it; NULL where memory is short (the
+// site transforms do without them).
+double2 *kubo_table_reserve(Session *s, int M, int nump) {
+  try {
+    return table_buffers(s, M, nump).table;
+  } catch (const Error &e) {
+    if (e.code != LINQT_ERR_NOMEM || s->strict_memory) throw;
+    s->release("kt_");
+    return nullptr;
+  }
+}
+
 // acc += what kubo_fft_sites gives (the parts of p and w that reach sigma), from the raw table
 // hi + lo [M][M].
 void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc) {
-  const int n = nump, A = best_split(M, n), P = 2 * n / A;
-  const int IB = std::max(1, std::min(P, kTabPairs / A));
-  const int blocks = (P + IB - 1) / IB;
-  const int groups = std::max(1, std::min(M, 4 * s->sm_count / blocks));
-  double2 *tab = (double2 *)s->get("kt_cos", sizeof(double2) * 4 * (size_t)n);
-  double *amp = (double *)s->get("kt_amp", sizeof(double) * (size_t)M);
-  double2 *re = (double2 *)s->get("kt_coef", sizeof(double2) * 2 * (size_t)M * M), *im = re + (size_t)M * M;
-  double2 *part = (double2 *)s->get("kubo_part", sizeof(double2) * 2 * (size_t)groups * (n + 1));
+  const int n = nump;
+  const TableGrid tg = table_grid(s, M, n);
+  const int A = tg.A, P = tg.P, IB = tg.IB, blocks = tg.blocks, groups = tg.groups;
+  const TableBuffers b = table_buffers(s, M, n);
+  double2 *tab = b.cosines, *re = b.coef, *im = re + (size_t)M * M, *part = b.part;
+  double *amp = b.amp;
   k_dd_cosines<<<(4 * n + 127) / 128, 128, 0, s->stream>>>(n, tab);
   LQ_LAUNCHED();
   k_amplitudes<<<(M + 127) / 128, 128, 0, s->stream>>>(M, amp);

@@ -325,21 +325,36 @@ void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 
   LQ_LAUNCHED();
 }
 
-const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, size_t planes,
+namespace {
+dim3 commit_grid(Session *s, int M, long K, bool moments, long *kchunk) {
+  const KSplit k = moments ? split_k(s, M, M, K) : KSplit{1, K};
+  *kchunk = k.kchunk;
+  return dim3((M + BN - 1) / BN, (M + BM - 1) / BM, (unsigned)k.S);
+}
+}  // namespace
+
+// The buffers of the FP64 kernel first: they are the ones that a solve cannot do without.
+int mu_reserve_rns(Session *s, int M, long K, bool moments) {
+  long kchunk = 0;
+  const dim3 grid = commit_grid(s, M, K, moments, &kchunk);
+  if (moments) s->get("zgemm_parts", sizeof(double2) * (size_t)grid.z * M * M);
+  s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
+  return rns_reserve(s, M, M, K);
+}
+
+const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int slab,
                            double2 *mu_raw, double2 *tab) {
   LQ_REQUIRE(!(fp32_inputs && mu_raw), "residues: moments of FP64 blocks only");
   const size_t MM = (size_t)M * M;
-  const KSplit k = mu_raw ? split_k(s, M, M, K) : KSplit{1, K};
-  const dim3 grid((M + BN - 1) / BN, (M + BM - 1) / BM, (unsigned)k.S);
-  double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MM) : nullptr;
+  long kchunk = 0;
+  const dim3 grid = commit_grid(s, M, K, mu_raw != nullptr, &kchunk);
+  double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)grid.z * MM) : nullptr;
   unsigned *tiles = (unsigned *)s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
-  double2 *sum = (double2 *)s->get("rns_sum", sizeof(double2) * 2 * MM);
-  const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, planes, sum, sum + MM);
+  const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
   const size_t smem = zgemm_smem(sizeof(double2));
   raise_smem_limit((const void *)k_commit, smem);
-  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, sum, sum + MM, (const double2 *)L,
-                                           (const double2 *)Rv, M, K, k.kchunk, part, tiles, mu_raw, tab,
-                                           tab ? tab + MM : nullptr);
+  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
+                                           M, K, kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr);
   LQ_LAUNCHED();
   return &j.stats->rejected;
 }
@@ -347,9 +362,9 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
                  double2 *mu_raw) {
   if (!fp32_inputs) {
-    const size_t planes = rns_faster(M, M, K) ? rns_plane_bytes(s, M, M, K) : 0;
-    if (planes)
-      (void)mu_contract_rns(s, L, Rv, M, K, false, planes, mu_raw, nullptr);
+    const int slab = rns_faster(M, M, K) ? mu_reserve_rns(s, M, K, true) : 0;
+    if (slab)
+      (void)mu_contract_rns(s, L, Rv, M, K, false, slab, mu_raw, nullptr);
     else
       zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
   } else if (i8_digits(precision)) {

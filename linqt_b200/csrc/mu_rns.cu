@@ -592,11 +592,6 @@ bool rns_faster(int MA, int MB, long K) {
   return m >= 160 ? K >= std::max(192, std::max(MA, MB)) : m >= 8 && K >= 192 && K <= 8192;
 }
 
-size_t rns_bytes(int MA, int MB, long K) {
-  const size_t per_k = (size_t)kPlanes * (MA + MB);
-  return per_k * (size_t)((K + kBk - 1) / kBk + K / kChunkMax + 1) * kBk;  // chunks are rounded up
-}
-
 // Time of the contraction here, us: 30 of launches, 13.5 ps an entry for the residues, the GEMMs of
 // the padded tiles at 2.4 POPS (fits the times above within 20 % at K >= 2048).
 double rns_us(int M, long K) {
@@ -604,49 +599,99 @@ double rns_us(int M, long K) {
   return 30 + 2.0 * M * K * 13.5e-6 + kPlanes * pad * pad * K * 2 / 2.4e9;
 }
 
-// Planes for a contraction here, allocated (0: not enough memory is left).
-size_t rns_plane_bytes(Session *s, int MA, int MB, long K) {
-  const size_t all = rns_bytes(MA, MB, K);
+namespace {
+// The split of K, from the sizes alone: kc values a chunk, the rows' exponents are of a chunk, so no
+// bit of a result depends on how many chunks' planes fit at a time.
+constexpr size_t kPlaneMax = 8ull << 30;  // one chunk's planes, at most
+struct RnsPlan {
+  int kc;
+  long chunks;
+  size_t planes, res, exps;  // bytes of one chunk
+  size_t chunk_bytes() const { return planes + res + exps; }
+};
+RnsPlan rns_plan(int MA, int MB, long K) {
   const size_t per_k = (size_t)kPlanes * (MA + MB);
-  const size_t least = per_k * (size_t)std::min(kPart, (int)((K + kBk - 1) / kBk) * kBk);
-  size_t want = std::min(s->rns_budget, all);
-  auto it = s->ws.find("rns_planes");  // memory is short: fewer chunks at a time, or the FP64 kernel
-  const size_t have = it == s->ws.end() ? 0 : it->second.second;
-  if (have >= want || s->capturing) return have >= least ? std::min(have, std::max(want, least)) : 0;
-  for (; want >= least; want /= 2) {
+  const long cap = std::max<long>(kBk, std::min<long>(kChunkMax, (long)(kPlaneMax / per_k) / kBk * kBk));
+  const long total = (K + cap - 1) / cap;
+  RnsPlan p;
+  p.kc = (int)(((K + total - 1) / total + kBk - 1) / kBk * kBk);
+  p.chunks = (K + p.kc - 1) / p.kc;
+  p.planes = per_k * p.kc;
+  p.res = (size_t)kPlanes * MA * ((MB + 15) / 16 * 16);
+  p.exps = sizeof(int) * (size_t)(MA + MB);
+  return p;
+}
+long slab_of(const RnsPlan &p, size_t budget) {
+  return std::max(1L, std::min(p.chunks, (long)(budget / p.planes)));
+}
+size_t held_bytes(const Session *s, const char *name) {
+  auto it = s->ws.find(name);
+  return it == s->ws.end() ? 0 : it->second.second;
+}
+}  // namespace
+
+// Bytes of a contraction here with planes of about `budget` bytes (one chunk's at least).
+size_t rns_footprint(int MA, int MB, long K, size_t budget) {
+  const RnsPlan p = rns_plan(MA, MB, K);
+  return slab_of(p, budget) * p.chunk_bytes() + sizeof(double2) * 2 * (size_t)MA * MB +
+         sizeof(RnsSide) * 2 * (size_t)p.chunks;
+}
+
+// Chunks of K at a time whose buffers the session holds from here on: all of them or none
+// (0: use the FP64 kernel).  What is held is used; where that is less than the budget allows, up to
+// half of the free memory is taken (or one chunk's), and less when that fails.  Only this call is
+// the worse for memory that is short now.  A served request that runs beside others fails instead, and runs
+// again alone (server.cu): its result must not depend on them.
+int rns_reserve(Session *s, int MA, int MB, long K) {
+  if (!s->rns_budget) return 0;
+  const RnsPlan p = rns_plan(MA, MB, K);
+  const size_t sum = sizeof(double2) * 2 * (size_t)MA * MB, sides = sizeof(RnsSide) * 2 * (size_t)p.chunks;
+  long want = slab_of(p, s->rns_budget);
+  long held = std::min({(long)(held_bytes(s, "rns_planes") / p.planes), (long)(held_bytes(s, "rns_res") / p.res),
+                        (long)(held_bytes(s, "rns_exp") / p.exps)});
+  if (held_bytes(s, "rns_sum") < sum || held_bytes(s, "mu_sides_counter") < sides || !held_bytes(s, "mu_judge_counter") ||
+      !held_bytes(s, "mu_tc_err_barrier"))
+    held = 0;
+  if (held >= want || s->capturing) return (int)std::min(held, want);
+  if (!s->hbm_budget) {
+    size_t room = free_pool_bytes(s->device);
+    for (const char *name : {"rns_planes", "rns_res", "rns_exp"}) room += held_bytes(s, name);
+    if (room < p.chunk_bytes()) return (int)held;
+    want = std::max(1L, std::min(want, (long)(room / 2 / p.chunk_bytes())));
+    if (want < 2 * held) return (int)held;  // not worth new buffers
+  }
+  for (; want; want /= 2) {
     try {
-      s->get("rns_planes", want);
-      return want;
+      s->get("rns_sum", sum);
+      s->get("mu_judge_counter", sizeof(RnsStats));  // "counter", "barrier": zeroed when allocated
+      s->get("mu_sides_counter", sides);
+      s->get("mu_tc_err_barrier", sizeof(int) * 4);
+      s->get("rns_exp", p.exps * want);
+      s->get("rns_res", p.res * want);
+      s->get("rns_planes", p.planes * want);
+      return (int)want;
     } catch (const Error &e) {
-      if (e.code != LINQT_ERR_NOMEM) throw;
-      s->rns_budget = want / 2;  // do not ask for as much again on every call
+      if (e.code != LINQT_ERR_NOMEM || s->strict_memory) throw;
+      s->release("rns_");
     }
   }
   return 0;
 }
 
-// sum (hi + lo, MA x MB) = sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K),
-// with planes of at most plane_bytes bytes at a time, and what it is to be judged by.
-RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs,
-                          size_t plane_bytes, double2 *sum_hi, double2 *sum_lo) {
-  // K chunks of equal length, a multiple of the GEMM block, short enough for one set of planes
-  const size_t per_k = (size_t)kPlanes * (MA + MB);
-  long cap = std::min<long>(kChunkMax, (long)(plane_bytes / per_k) / kBk * kBk);
-  cap = std::max<long>(cap, kBk);
-  const long total = (K + cap - 1) / cap;
-  const int kc = (int)(((K + total - 1) / total + kBk - 1) / kBk * kBk);
-  const long nchunk_all = (K + kc - 1) / kc;
-  const int nkb = kc / kBk;
-  const int slab = (int)std::max(1L, std::min(nchunk_all, (long)(plane_bytes / (per_k * kc))));
-  const int pitch = (MB + 15) / 16 * 16;
-  int8_t *plA = (int8_t *)s->get("rns_planes", per_k * (size_t)kc * slab);
+// sum (hi + lo, MA x MB) = sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K), `slab`
+// chunks at a time (rns_reserve), and what it is to be judged by.
+RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab) {
+  const RnsPlan p = rns_plan(MA, MB, K);
+  const int kc = p.kc, nkb = kc / kBk, pitch = (MB + 15) / 16 * 16;
+  double2 *sum_hi = (double2 *)s->get("rns_sum", sizeof(double2) * 2 * (size_t)MA * MB);
+  double2 *sum_lo = sum_hi + (size_t)MA * MB;
+  int8_t *plA = (int8_t *)s->get("rns_planes", p.planes * slab);
   int8_t *plB = plA + (size_t)kPlanes * MA * kc * slab;
-  uint8_t *res = (uint8_t *)s->get("rns_res", (size_t)slab * kPlanes * MA * pitch);
-  int *eA = (int *)s->get("rns_exp", sizeof(int) * (size_t)(MA + MB) * slab);
+  uint8_t *res = (uint8_t *)s->get("rns_res", p.res * slab);
+  int *eA = (int *)s->get("rns_exp", p.exps * slab);
   int *eB = eA + (size_t)MA * slab;
-  // "counter": zeroed when they are allocated
   RnsStats *stats = (RnsStats *)s->get("mu_judge_counter", sizeof(RnsStats));
-  RnsSide *side = (RnsSide *)s->get("mu_sides_counter", sizeof(RnsSide) * 2 * (size_t)nchunk_all);
+  RnsSide *side = (RnsSide *)s->get("mu_sides_counter", sizeof(RnsSide) * 2 * (size_t)p.chunks);
   int *err = (int *)s->get("mu_tc_err_barrier", sizeof(int) * 4);  // read by mu_tc_check_error
   s->barrier_used = true;
   const CUtensorMap ta = make_map_rns(plA, MA, (long)nkb * kPlanes * slab),
@@ -654,8 +699,8 @@ RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int 
   const int parts = (kc + kPart - 1) / kPart;  // 8 at most
   const size_t smem = sizeof(RnsShared) + 1024;
   raise_smem_limit((const void *)k_rns_gemm, smem);
-  for (long c0 = 0; c0 < nchunk_all; c0 += slab) {
-    const int nc = (int)std::min<long>(slab, nchunk_all - c0);
+  for (long c0 = 0; c0 < p.chunks; c0 += slab) {
+    const int nc = (int)std::min<long>(slab, p.chunks - c0);
     const long k0 = c0 * kc, len = std::min(K - k0, (long)nc * kc);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(parts, std::max(MA, MB), 2 * nc);
@@ -678,11 +723,11 @@ RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int 
     k_rns_gemm<<<2 * pairs, kRnsThreads, smem, s->stream>>>(ta, tb, MA, MB, len, kc, nkb, nc, res, pitch, err);
     LQ_LAUNCHED();
     const int g = (int)std::max(1L, std::min(((long)MA * MB + 255) / 256, (long)s->sm_count * 8));
-    k_rns_crt<<<g, 256, 0, s->stream>>>(res, pitch, MA, MB, nc, eA, eB, c0 == 0, c0 + nc == nchunk_all,
+    k_rns_crt<<<g, 256, 0, s->stream>>>(res, pitch, MA, MB, nc, eA, eB, c0 == 0, c0 + nc == p.chunks,
                                         stats, sum_hi, sum_lo);
     LQ_LAUNCHED();
   }
-  return {stats, side, (int)nchunk_all};
+  return {sum_hi, sum_lo, stats, side, (int)p.chunks};
 }
 
 // After a wait that expired: the statistics of the contractions so far are void.

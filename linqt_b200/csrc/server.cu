@@ -51,7 +51,7 @@ struct Job {
   void *states = nullptr;  // pinned host copy (server pool); NULL: generated on the device
   size_t states_cap = 0;
   size_t footprint = 0;
-  size_t rns_budget = 0;  // residue planes, part of the footprint
+  size_t rns_budget = 0;  // residue planes, part of the footprint (0: none)
   int block_width = 1;
   int status = 0;  // 0 pending, 1 running, 2 done, <0 error
   bool alone = false;  // ran out of memory next to other requests: runs again with none beside it
@@ -208,6 +208,7 @@ struct linqt_server {
           const size_t sb = sizeof(double2) * (size_t)R * n;
           const size_t mb = sizeof(double2) * (size_t)M * (job->req.kind == LINQT_REQ_DOS ? 1 : M);
           s.rns_budget = job->rns_budget;
+          s.strict_memory = !job->alone;
           s.hbm_budget = job->footprint;  // fixed per request: chunking independent of the other requests
           double2 *d_st = (double2 *)s.get("io_states", sb);
           double2 *d_mu = (double2 *)s.get("io_mu", mb);
@@ -324,11 +325,12 @@ int linqt_server_submit(linqt_server *srv, const linqt_request *req, long *ticke
     // planes for the contraction in residues (the FP64 moments', and sigma's) where the budget
     // has room for them and for the tables of sigma; else the request runs without them
     if (req->kind == LINQT_REQ_KUBO_BASTIN && (req->precision == LINQT_PREC_FP64 || req->sigma_out)) {
-      const size_t planes = std::min(rns_bytes(req->M, req->M, (long)n * job->block_width), (size_t)2 << 30);
-      const size_t tables = sizeof(double2) * 8 * (size_t)req->M * req->M;
-      if (job->footprint + planes + tables <= srv->budget) {
+      const size_t planes = (size_t)2 << 30;
+      const size_t more = rns_footprint(req->M, req->M, (long)n * job->block_width, planes) +
+                          sizeof(double2) * 8 * (size_t)req->M * req->M;
+      if (job->footprint + more <= srv->budget) {
         job->rns_budget = planes;
-        job->footprint += planes + tables;
+        job->footprint += more;
       }
     }
     if (job->footprint > srv->budget)
