@@ -3,6 +3,7 @@
 // Every entry point catches linqt::Error (and std::exception) and turns it into a
 // negative status plus a thread-local message; nothing aborts across the ABI.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -65,8 +66,12 @@ void *Session::get(const std::string &name, size_t bytes) {
     e = cudaMallocAsync(&p, bytes, stream);
   };
   if (e == cudaErrorMemoryAllocation) retry();
-  // the residue planes are an option (mu_rns.cu): they give way to any other buffer
-  if (e == cudaErrorMemoryAllocation && name.rfind("rns_", 0) != 0 && release("rns_")) retry();
+  // the residue planes (mu_rns.cu) and the buffers of sigma's table (kubo_table.cu), while no solve
+  // uses them, are an option: they give way to any other buffer
+  if (e == cudaErrorMemoryAllocation && name.rfind("rns_", 0) != 0 && name.rfind("kt_", 0) != 0) {
+    const bool planes = release("rns_"), tables = !table_in_use && release("kt_");
+    if (planes || tables) retry();
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(LINQT_ERR_NOMEM, "cudaMallocAsync(" + std::to_string(bytes) + ") for '" + name + "' failed: " +
@@ -892,8 +897,15 @@ static long lr_vectors(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   return launches;
 }
 
+// The width and number of the vector chunks of a solve.  A solve that has been enqueued notes its sizes and
+// width in the session (done), for the next of the same sizes.
 struct Chunking {
   int Rc, nchunks;
+  std::array<size_t, 7> sizes;
+  void done(Session *s) const {
+    s->chunk_sizes = sizes;
+    s->chunk_width = Rc;
+  }
 };
 
 // pick the vector-chunk width so that 2 stores of M*N*Rc + buffers fit in memory, with the
@@ -903,6 +915,23 @@ static Chunking pick_chunks(Session *s, int N, int R, int M, size_t esz, const l
                             int digits = 0) {
   int Rc = o.block_width > 0 ? pow2_at_least(o.block_width) : pow2_at_least(R);
   Rc = std::min(Rc, 256);
+  const std::array<size_t, 7> sizes = {(size_t)N, (size_t)R, (size_t)M, esz, (size_t)o.block_width, extra, (size_t)digits};
+  const auto chunks = [&](int rc) { return Chunking{rc, (R + rc - 1) / rc, sizes}; };
+  // What the last solve fitted in still fits where its blocks are still held, whatever else has been
+  // allocated since: the same call gets the same width, and at full width the device need not be
+  // asked for its free memory (which takes longer than the smaller solves).
+  const size_t blk = esz * (size_t)N;
+  const auto held = [&](const char *name) {
+    auto it = s->ws.find(name);
+    return it == s->ws.end() ? 0 : it->second.second;
+  };
+  int kept = 0;
+  if (!s->hbm_budget && s->chunk_width && s->chunk_sizes == sizes) {
+    const size_t b = blk * s->chunk_width;
+    if (held("lr_L") >= b * M && held("lr_R") >= b * M && held("lr_tmp") >= 4 * b) kept = s->chunk_width;
+  }
+  s->chunk_width = 0;  // until this solve is enqueued
+  if (kept == Rc) return chunks(Rc);
   size_t avail;
   if (s->hbm_budget) {
     // a session with a fixed budget (serving) chunks by the budget alone, so the
@@ -911,25 +940,27 @@ static Chunking pick_chunks(Session *s, int N, int R, int M, size_t esz, const l
   } else {
     avail = free_device_bytes();
     // plus what this session already holds in the buffers this solve reallocates (the L/R
-    // stores and the digit planes); its other cached workspaces stay allocated
+    // stores and the digit planes) or can do without (residue planes, sigma's table); its other
+    // cached workspaces stay allocated
     for (auto &kv : s->ws)
-      if (kv.first.rfind("lr_", 0) == 0 || kv.first.rfind("mu_i8_", 0) == 0) avail += kv.second.second;
+      for (const char *p : {"lr_", "mu_i8_", "rns_", "kt_"})
+        if (kv.first.rfind(p, 0) == 0) avail += kv.second.second;
     avail = (size_t)(avail * 0.90);
   }
   // the Chebyshev blocks (L and R stores, 4 scratch blocks) and, for the INT8 contraction,
   // one K slab of digit planes
   const auto need_at = [&](int rc) {
-    return esz * (size_t)N * rc * (2 * (size_t)M + 4) + extra + i8_digit_bytes(digits, M, (long)N * rc);
+    return blk * rc * (2 * (size_t)M + 4) + extra + i8_digit_bytes(digits, M, (long)N * rc);
   };
-  while (Rc > 1) {
+  while (Rc > std::max(1, kept)) {
     if (need_at(Rc) <= avail) break;
     Rc >>= 1;
   }
   const size_t need = need_at(Rc);
-  if (need > avail)
+  if (need > avail && Rc != kept)
     fail(LINQT_ERR_NOMEM, "2D moments: " + std::to_string(need >> 20) + " MiB of Chebyshev blocks exceed the " +
                               std::to_string(avail >> 20) + " MiB available");
-  return {Rc, (R + Rc - 1) / Rc};
+  return chunks(Rc);
 }
 
 // Whether the vector blocks are FP32 (the operators stay FP64 in every mode).
@@ -972,6 +1003,7 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
   PhaseScope ph(s, PH_OTHER);
   mu_finalize(s, raw, M, R, mu);
   ph.launches(1);
+  ch.done(s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1019,6 +1051,10 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   char *Rs = (char *)s->get("lr_R", blk * M);
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
   double2 *raw = nullptr, *acc = nullptr, *acc_c = nullptr, *tab = nullptr;
+  struct TableUse {
+    Session *s;
+    ~TableUse() { s->table_in_use = false; }
+  } table_use{s};
   const size_t MM = (size_t)M * M;
   if (mu) {
     raw = (double2 *)s->get("mu_raw", sizeof(double2) * MM);
@@ -1041,6 +1077,7 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     if (s->rns_budget &&
         kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
       tab = kubo_table_reserve(s, M, nump);
+    s->table_in_use = tab != nullptr;
     if (tab) LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
   }
   for (int c = 0; c < ch.nchunks; ++c) {
@@ -1084,6 +1121,7 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
   if (mu) mu_finalize(s, raw, M, R, mu);
   if (out) kubo_postprocess(s, acc, R, nump, formula, N, bw, bc, out);
   ph.launches((mu ? 1 : 0) + (out ? 1 : 0));
+  ch.done(s);
 }
 
 // ---------------------------------------------------------------------------

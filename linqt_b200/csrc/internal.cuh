@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <condition_variable>
 #include <cstdint>
 #include <map>
@@ -274,6 +275,9 @@ struct Session {
   size_t hbm_budget = 0;  // chunking budget; 0 = what the device has free
   size_t rns_budget = 8ull << 30;  // residue planes of the FP64 contraction (mu_rns.cu); 0: none
   bool strict_memory = false;      // an optional buffer that does not fit fails the solve (served beside others)
+  bool table_in_use = false;       // by the solve being enqueued: its "kt_" workspaces stay
+  std::array<size_t, 7> chunk_sizes{};  // of the last 2D solve enqueued, and its vector chunks' width (api.cu)
+  int chunk_width = 0;
   bool barrier_used = false;  // a persistent kernel ran since the last error check
   // fault injection for tests (linqt_session_inject_barrier_timeout): grid barriers await
   // inject_extra more CTAs than launched and give up after inject_limit polls

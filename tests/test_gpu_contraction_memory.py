@@ -1,6 +1,7 @@
 """FP64 solves when the device has little memory left: the residue planes of the contraction are an
-option, never what a solve fails for, and only the call that runs short of memory is the worse for it.
-A torch buffer takes the rest of the device."""
+option, never what a solve fails for, only the call that runs short of memory is the worse for it, and the
+same call gives the same blocks and bits whatever planes an earlier one has left in the session.  A
+torch buffer takes the rest of the device."""
 import contextlib
 
 import numpy as np
@@ -84,6 +85,14 @@ def test_a_call_repeats_its_blocks_and_bits(solve, wanted, session):
     assert np.array_equal(solve(session), wanted[0])
 
 
+def test_planes_left_behind_do_not_narrow_the_next_solve(solve, wanted, session):
+    """A session that holds planes from a solve with room for them, and then the device fills up."""
+    assert np.array_equal(solve(session), wanted[0])
+    with only(int(0.2e9)):
+        assert np.array_equal(solve(session), wanted[0])
+        assert np.array_equal(solve(session, precision=lq.PREC_MIXED), wanted[2])
+
+
 @pytest.mark.parametrize("sigma", [False, True])
 def test_no_size_of_the_rest_fails(solve, wanted, sigma):
     """The planes may take the rest of the memory, or nearly, but not what the solve needs besides."""
@@ -111,3 +120,23 @@ def test_a_served_request_does_not_change_kernels_for_its_neighbours(solve):
             assert srv.retries()[1] == 1
     finally:
         srv.close()
+
+
+def test_a_solve_that_just_fits_is_not_refused_the_second_time(solve):
+    """One vector a block: what the arithmetic leaves after the first call is less than before it."""
+    n, H, V = lattices.honeycomb(256, 256, t=-2.7, W=1.0, seed=21)
+    Hg, Vg = lq.Operator.from_csr(n, *H), lq.Operator.from_csr(n, *V)
+    Hg.rescale_to_chebyshev(BW, 0.0)
+    st = torch.from_numpy(lattices.random_phase_states(n, 1, seed=4).view(np.float64)).cuda()
+    mu = torch.zeros(2 * M * M, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    blocks = 16 * n * (2 * M + 4) + 16 * 66 * M * M  # what a solve counts
+    session = lq.Session(0)
+    with only(int(blocks / 0.9) + (48 << 20)):
+        got = []
+        for _ in range(4):
+            lq.moments2d_dev(Hg, Vg, Vg, st, 1, M, mu, session=session)
+            session.synchronize()
+            got.append(mu.cpu().numpy().copy())
+    session.close()
+    assert all(np.array_equal(g, got[0]) for g in got)
