@@ -641,6 +641,10 @@ size_t max_slice_bytes(const DeviceOp &H, const DeviceOp *V, int grid, size_t es
   return worst;
 }
 
+// CTAs of `full` that a share of the device covers.  A grid of n CTAs asks for n / full, whose product
+// with full may fall short of n in FP64.
+long share_ctas(double full, double share) { return std::max(1L, (long)(full * share + 1e-6)); }
+
 // Cooperative grid: as many co-resident CTAs as fit (at most one CTA's worth of rows per
 // group of TPR threads).  The operator slices are cached in shared memory when they fit.
 int coop_setup(Session *s, const void *func, const DeviceOp &H, const DeviceOp *V, int tpr, size_t esz,
@@ -653,7 +657,7 @@ int coop_setup(Session *s, const void *func, const DeviceOp &H, const DeviceOp *
   const double share = coop_share_take(s, std::min(1.0, (double)need / ((double)per_sm * sm_count)));
   // a session with an SM share (linqt_session_set_sm_share) keeps its grid to that fraction
   // of the co-resident CTAs, so that grids of sessions whose shares add up to 1 fit together
-  const auto cap = [&](int p) { return std::max(1L, (long)(p * (double)sm_count * share)); };
+  const auto cap = [&](int p) { return share_ctas((double)p * sm_count, share); };
   const int grid0 = (int)std::max(1L, std::min(cap(per_sm), need));
   const size_t limit = 96 * 1024;
   // 96 KB for every launch of these kernels, whichever thread launches them
@@ -688,8 +692,7 @@ int coop_grid(Session *s, const void *func, long max_blocks, size_t smem) {
   if (per_sm <= 0) fail(LINQT_ERR_UNSUPPORTED, "persistent kernel does not fit on an SM");
   const double full = (double)per_sm * s->sm_count;
   const double share = coop_share_take(s, std::min(1.0, (double)max_blocks / full));
-  const long cap = std::max(1L, (long)(full * share));
-  return (int)std::max(1L, std::min(cap, max_blocks));
+  return (int)std::max(1L, std::min(share_ctas(full, share), max_blocks));
 }
 
 double coop_share_take(Session *s, double want) {
