@@ -407,7 +407,7 @@ static void require_c128_operators(const linqt_opts &o, const char *who) {
 // opts.use_graphs: a *_dev solve is enqueued eagerly on its first call with a given key (so
 // that every workspace is allocated and any autotuning is done), captured into a CUDA graph
 // on the second and replayed from the instantiated graph afterwards.  The key holds every
-// pointer and size of the call and the operators' upload ids and versions; a workspace
+// pointer, size and option of the call and the operators' upload ids and versions; a workspace
 // reallocation drops all graphs of the session.  While capturing, cooperative launches go on
 // the session stream itself rather than the device lane.  Sessions on the legacy default
 // stream, sessions with phase timing on, and keys whose capture failed run eagerly.
@@ -429,7 +429,8 @@ static std::string call_key(const char *name, std::initializer_list<const void *
     snprintf(buf, sizeof(buf), ":%a", x);
     k += buf;
   }
-  snprintf(buf, sizeof(buf), ":%d.%d.%d.%d.%d", o.precision, o.format, o.block_width, o.doubling, o.step_launches);
+  snprintf(buf, sizeof(buf), ":%d.%d.%d.%d.%d.%d.%d.%d", o.precision, o.format, o.block_width, o.doubling,
+           o.step_launches, o.realisations, o.operator_precision, o.thread_shape);
   return k + buf;
 }
 
