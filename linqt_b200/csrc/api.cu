@@ -486,14 +486,16 @@ static void with_graph(Session *s, const linqt_opts &o, const std::string &key, 
 // for every layout (CSR cached, CSR uncached, SELL with C = 8 and 32, and on large blocks
 // the two locality layouts) and thread shape, keeps the fastest per
 // operator pair, block width and precision, and returns it.  Each candidate runs once
-// untimed (building its layout) and once timed.
+// untimed (building its layout) and once timed.  on_chip: the cached CSR layout runs in the kernels
+// of small blocks, which have no thread shapes, and is timed once.
 // ---------------------------------------------------------------------------
 struct RecCfg {
   int sellC = 0, shape = 0;
 };
 
 static RecCfg pick_layout(Session *s, const DeviceOp &H, const std::string &key, int format, int Rc, int shape,
-                          const std::function<void(int, int)> &trial, float *best_ms = nullptr) {
+                          const std::function<bool()> &on_chip, const std::function<void(int, int)> &trial,
+                          float *best_ms = nullptr) {
   if (best_ms) *best_ms = -1;
   if (format == LINQT_FORMAT_CSR) return RecCfg{0, shape};
   if (format == LINQT_FORMAT_SELL || format == LINQT_FORMAT_LOCAL) {
@@ -516,10 +518,11 @@ static RecCfg pick_layout(Session *s, const DeviceOp &H, const std::string &key,
   // copied in the locality order) and 32 | kSellLocality: tried when one block of the lattice
   // (8 bytes per value at least) exceeds 64 MB, i.e. when its neighbour rows can leave L2
   // between their reads
-  const bool big = (double)H.n * Rc * sizeof(float2) > 64e6;
+  const bool big = (double)H.n * Rc * sizeof(float2) > 64e6, chip = on_chip();
   for (int C : {0, -1, 8, 32, 1 | kSellLocality, 32 | kSellLocality})
     for (int sh = 0; sh < recur_shapes(Rc); ++sh) {
       if ((C & kSellLocality) && !big) continue;
+      if (C == 0 && chip && sh > 0) continue;
       trial(C, sh);
       LQ_CUDA(cudaEventRecord(a, s->stream));
       trial(C, sh);
@@ -567,6 +570,9 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
   char *T = (char *)s->get("m1_T", 3 * esz * (size_t)N * Rc);
   PhaseScope ph(s, PH_RECURSION);
   long launches = 0;
+  // a thread shape asked for leaves the on-chip kernels out, and is tuned by itself
+  const bool chip = o.thread_shape == 0;
+  const std::string asked = chip ? "" : ":shape";
   const auto shape_of = [&](int w) {
     return recur_default_shape((long)N * w, w, fp32, o.format == LINQT_FORMAT_LOCAL);
   };
@@ -576,7 +582,8 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
     const int Mt = std::min(M, 32), st = doubling ? (Mt + 1) / 2 : Mt;
     double2 *tdots = (double2 *)s->get("m1_trial_dots", sizeof(double2) * 2 * (size_t)st);
     return pick_layout(
-        s, H, layout_key(c64 ? "1d64" : "1d", op, w, fp32), o.format, w, shape_of(w),
+        s, H, layout_key(c64 ? "1d64" : "1d", op, w, fp32) + asked, o.format, w, shape_of(w),
+        [&] { return chip && !c64 && recur_1d_on_chip(s, H, w, fp32); },
         [&](int C, int shape) {
           // a short recursion on the first chunk (the real run below starts from scratch)
           void *b0 = T, *b1 = T + bw, *b2 = T + 2 * bw;
@@ -589,7 +596,7 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
               LQ_CUDA(cudaMemcpyAsync(b0, b2, bw, cudaMemcpyDeviceToDevice, s->stream));
             x0 = b0;
           }
-          recur_1d(s, H, b2, x0, b1, st, Mt, doubling ? 2 : 1, w, fp32, tdots, C, shape, nullptr, 1, c64);
+          recur_1d(s, H, b2, x0, b1, st, Mt, doubling ? 2 : 1, w, fp32, tdots, C, shape, nullptr, 1, c64, chip);
         },
         best_ms);
   };
@@ -599,7 +606,7 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
   if (o.format == LINQT_FORMAT_AUTO && o.block_width <= 0 && !o.step_launches && Rc > 1) {
     DeviceOp &Hm = const_cast<DeviceOp &>(H);
     const std::string wkey = "1dw:" + std::to_string(R) + ":" + layout_key(c64 ? "c64" : "", op, Rc, fp32) +
-                             (doubling ? ":d" : "");
+                             (doubling ? ":d" : "") + asked;
     int w = 0;
     {
       std::lock_guard<std::mutex> g(Hm.mu);
@@ -653,7 +660,7 @@ static void moments1d_dev(Session *s, const DeviceOp &H, const DeviceOp *op, con
         x0 = b0;
       }
       recur_1d(s, H, phi, x0, b1, steps, M, doubling ? 2 : 1, Rc, fp32, cd, cfg.sellC, cfg.shape, nullptr, 1, c64,
-               o.thread_shape == 0);
+               chip);
       launches += 2;
       continue;
     }
@@ -837,7 +844,9 @@ static long lr_vectors(Session *s, const DeviceOp &H, const DeviceOp *opl, const
       if (!opr) LQ_CUDA(cudaMemcpyAsync(Rstore, phi, blk, cudaMemcpyDeviceToDevice, s->stream));
     };
     const RecCfg cfg = pick_layout(s, H, layout_key("lr", opr, Rc, fp32), format, Rc,
-                                   recur_lr_default_shape((long)H.n * Rc, Rc, fp32), [&](int C, int shape) {
+                                   recur_lr_default_shape((long)H.n * Rc, Rc, fp32),
+                                   [&] { return cluster_recur_lr(s, H, opr, nullptr, nullptr, nullptr, M, Rc, fp32); },
+                                   [&](int C, int shape) {
       start();
       recur_lr(s, H, opr, Lstore, Rstore, phi, tmp3, std::min(M, 16), Rc, fp32, C, shape);
     });

@@ -475,7 +475,10 @@ void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1
               bool c64 = false, bool on_chip = true);
 // dots[(r*steps + s)*2 + i] = sums of partials[steps][nb][2] over the nb / nreal CTAs of each realisation
 void reduce_step_partials(Session *s, const double2 *partials, int steps, int nb, int nreal, double2 *dots);
-// the same recursions of small lattices in one cluster (recur_cluster.cu); false: too large
+// whether recur_1d runs the cached CSR layout of a block on chip: in one cluster or from registers
+bool recur_1d_on_chip(Session *s, const DeviceOp &H, int R, bool fp32);
+// the same recursions of small lattices in one cluster (recur_cluster.cu); false: too large.  With
+// dots or Lst NULL they only ask.
 constexpr int kRegsRow = 16;  // k_recur_1d_regs: entries of the longest row it takes
 bool cluster_recur_1d(Session *s, const DeviceOp &H, const void *phi, const void *x0, int steps, int M, int mode, int R,
                       bool fp32, double2 *dots);

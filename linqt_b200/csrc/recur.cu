@@ -1000,7 +1000,7 @@ void recur_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lstore, vo
 }
 
 namespace {
-// False if the threads of a cooperative grid do not cover the block.
+// False if the threads of a cooperative grid do not cover the block.  dots NULL: only asks.
 template <class T, int NR, int MINB>
 bool run_1d_regs(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
                  double2 *dots) {
@@ -1010,6 +1010,7 @@ bool run_1d_regs(Session *s, const DeviceOp &H, const void *phi, void *x0, void 
   int per_sm = 0;
   LQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kThreads, 0));
   if (need > (long)per_sm * s->sm_count) return false;
+  if (!dots) return true;
   const int grid = coop_grid(s, f, need, 0);
   if (grid < need) {  // a session with a share of the device
     coop_share_return(s);
@@ -1052,6 +1053,12 @@ bool recur_1d_regs(Session *s, const DeviceOp &H, const void *phi, void *x0, voi
   return false;
 }
 }  // namespace
+
+bool recur_1d_on_chip(Session *s, const DeviceOp &H, int R, bool fp32) {
+  return cluster_recur_1d(s, H, nullptr, nullptr, 1, 1, 1, R, fp32, nullptr) ||
+         (fp32 ? recur_1d_regs<float>(s, H, nullptr, nullptr, nullptr, 1, 1, 1, R, nullptr)
+               : recur_1d_regs<double>(s, H, nullptr, nullptr, nullptr, 1, 1, 1, R, nullptr));
+}
 
 void recur_1d(Session *s, const DeviceOp &H, const void *phi, void *x0, void *b1, int steps, int M, int mode, int R,
               bool fp32, double2 *dots, int sellC, int shape, const void *stacked, int nreal, bool c64,

@@ -369,6 +369,7 @@ bool run_1d(Session *s, const DeviceOp &H, const void *phi, const void *x0, int 
   using C = typename cplx_t<T>::type;
   const ClGeom g = cluster_geometry(s, (const void *)k_cluster_1d<T>, H, nullptr, R, sizeof(C), 2);
   if (!g.ctas) return false;
+  if (!dots) return true;
   const int nb = g.ctas * (g.threads / 32);
   double2 *partials = (double2 *)s->get("rec1d_part", sizeof(double2) * 2 * (size_t)steps * nb);
   cluster_launch(s, k_cluster_1d<T>, g, H.n, g.rshift, g.per, H.d_rowptr, H.d_col, H.d_val64, (const C *)phi,
@@ -383,6 +384,7 @@ bool run_lr(Session *s, const DeviceOp &H, const DeviceOp *V, void *Lst, void *R
   auto *f = V ? k_cluster_lr<T, true> : k_cluster_lr<T, false>;
   const ClGeom g = cluster_geometry(s, (const void *)f, H, V, R, sizeof(C), 4);
   if (!g.ctas) return false;
+  if (!Lst) return true;
   cluster_launch(s, f, g, H.n, g.rshift, g.per, H.d_rowptr, H.d_col, H.d_val64, V ? V->d_rowptr : nullptr,
                  V ? V->d_col : nullptr, V ? V->d_val64 : nullptr, (C *)Lst, (C *)Rst, (const C *)phi, M,
                  (size_t)H.n * R);
