@@ -14,6 +14,8 @@
 //
 // Arithmetic is that of recur.cu, entry by entry in the same order, so the blocks are the same
 // bits; the 1D moments differ by the order of the dot products' partial sums.
+#include <tuple>
+
 #include "internal.cuh"
 
 namespace linqt {
@@ -22,6 +24,7 @@ namespace {
 
 constexpr int kClMax = 16;          // CTAs of a cluster at most (above 8: opt-in)
 constexpr int kClThreads = 1024;    // threads of a CTA at most
+constexpr size_t kClSmem = 227 * 1024;  // dynamic shared memory of a CTA at most
 constexpr int kClItems = 128;       // values of a block per CTA at least (32 and 256 measure the same)
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
@@ -314,6 +317,34 @@ size_t op_slice_bytes(const DeviceOp &A, int r0, int r1) {
 // 1.70 / 1.91, 14400 x 1 (72k) 2.03 / 1.93; cubic 8000 x 1 (56k) 1.86 / 2.15, 10648 x 1 (75k) 2.26 / 2.15.
 constexpr long kClGathers1d = 80000, kClGathersRegs = 65000, kClGathersLr = 140000;
 
+// Whether the device can hold one cluster of `ctas` CTAs of func at the largest shared memory and thread
+// count that cluster_geometry gives (a device with fewer SMs a GPC, or a part of one, may not).  Asked
+// once per device, kernel and size.
+bool cluster_fits(int device, const void *func, int ctas) {
+  static std::mutex m;
+  static std::map<std::tuple<int, const void *, int>, bool> known;
+  std::lock_guard<std::mutex> g(m);
+  const auto key = std::make_tuple(device, func, ctas);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  raise_smem_limit(func, kClSmem);
+  bool ok = cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = kClSmem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  ok = ok && cudaOccupancyMaxActiveClusters(&n, func, &cfg) == cudaSuccess && n > 0;
+  if (!ok) cudaGetLastError();
+  return known[key] = ok;
+}
+
 ClGeom cluster_geometry(Session *s, const void *func, const DeviceOp &H, const DeviceOp *V, int R, size_t esz,
                         int blocks) {
   ClGeom g;
@@ -322,7 +353,6 @@ ClGeom cluster_geometry(Session *s, const void *func, const DeviceOp &H, const D
   const long items = (long)H.n * R;
   const long line = blocks == 4 ? kClGathersLr : blocks == 2 && H.max_row <= kRegsRow ? kClGathersRegs : kClGathers1d;
   if ((blocks == 4 ? 2 * H.nnz + (V ? V->nnz : 0) : H.nnz) * R > line) return g;
-  const size_t limit = 227 * 1024;
   while ((1 << g.rshift) < R) ++g.rshift;
   const int want = (int)std::min<long>(kClMax, std::max<long>(1, (items + kClItems - 1) / kClItems));
   int c = 1;
@@ -335,9 +365,8 @@ ClGeom cluster_geometry(Session *s, const void *func, const DeviceOp &H, const D
       worst = std::max(worst, op_slice_bytes(H, r0, r1) + (V ? op_slice_bytes(*V, r0, r1) : 0));
     }
     const size_t bytes = worst + (size_t)blocks * esz * ((size_t)per << g.rshift);
-    if (bytes > limit) continue;
-    raise_smem_limit(func, bytes);
-    LQ_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    if (bytes > kClSmem) continue;
+    if (!cluster_fits(s->device, func, c)) break;  // the grid kernels take it
     g.ctas = c;
     g.per = per;
     g.smem = bytes;
