@@ -406,7 +406,6 @@ inline size_t i8_digit_bytes(int digits, int M, long K) {
 
 // FFT path: accumulate p/w over all sites into acc[2*nump] (complex)
 // prefactors pf_m of Kubo_solver_FFT (kubo_fft.cu)
-void kubo_prefactors(Session *s, int M, int nump, double2 *pf);
 // only_if: acc += them, on the device where *only_if is set
 void kubo_fft_sites(Session *s, const void *L, const void *Rv, long nsites, int M, int nump, int formula,
                     bool fp32_inputs, double2 *acc, const int *only_if = nullptr);

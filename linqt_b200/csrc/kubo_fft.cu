@@ -151,8 +151,9 @@ __device__ __forceinline__ void greenwood_product(const double2 *X, int stride, 
   p.x += rb.x * rk.x + ib.x * ik.x;
 }
 
-// prefactors pf_m (src/Bastin_FFTs.cpp:20-21, include/Kubo_solver_FFT.hpp:99-107)
-__global__ void k_prefactors(int M, int nump, double2 *__restrict__ pf) {
+// prefactors pf_m (src/Bastin_FFTs.cpp:20-21, include/Kubo_solver_FFT.hpp:99-107), and for the direct
+// transforms the roots of unity tw
+__global__ void k_prefactors(int M, int nump, double2 *__restrict__ pf, double2 *__restrict__ tw) {
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     const double g = 1 / (M + 1.0) *
                      ((M - m + 1.0) * cos(M_PI * m / (M + 1.0)) + sin(M_PI * m / (M + 1.0)) / tan(M_PI / (M + 1.0)));
@@ -160,6 +161,12 @@ __global__ void k_prefactors(int M, int nump, double2 *__restrict__ pf) {
     double sn, cs;
     sincos(M_PI * m / (2.0 * nump), &sn, &cs);
     pf[m] = make_double2(amp * cs, amp * sn);
+  }
+  if (!tw) return;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nump; t += gridDim.x * blockDim.x) {
+    double sn, cs;
+    sincospi(2.0 * t / nump, &sn, &cs);
+    tw[t] = make_double2(cs, sn);
   }
 }
 
@@ -430,14 +437,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void k_twiddles(int n, double2 *__restrict__ tw) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * t / n, &sn, &cs);
-    tw[t] = make_double2(cs, sn);
-  }
-}
-
 // acc[t] = sum_b part[b][t]: 32 outputs a CTA, 8 threads each striding over b, then in order (one
 // thread per output: 107 us for 592 CTAs' partials).  only_if: acc += it where *only_if is set.
 __global__ void __launch_bounds__(256)
@@ -531,11 +530,8 @@ void launch_fft(Session *s, const Tin *L, const Tin *Rv, long K, int M, const do
 }
 
 template <int NSEQ, class Tin>
-void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump, const double2 *pf, double2 *acc,
-                const int *only_if) {
-  double2 *tw = (double2 *)s->get("kubo_tw", sizeof(double2) * nump);
-  k_twiddles<<<(nump + 255) / 256, 256, 0, s->stream>>>(nump, tw);
-  LQ_LAUNCHED();
+void launch_dft(Session *s, const Tin *L, const Tin *Rv, long K, int M, int nump, const double2 *pf,
+                const double2 *tw, double2 *acc, const int *only_if) {
   const size_t smem = sizeof(double2) * 2 * (size_t)M;
   if (smem > 227 * 1024) fail(LINQT_ERR_UNSUPPORTED, "kubo_fft: M too large for the direct DFT");
   raise_smem_limit((const void *)k_kubo_dft<NSEQ, Tin>, smem);
@@ -555,7 +551,7 @@ bool shared_memory_fft(int nump, int formula) {
 
 template <class Tin>
 void kubo_fft_sites_t(Session *s, const Tin *L, const Tin *Rv, long nsites, int M, int nump, int formula,
-                      const double2 *pf, double2 *acc, const int *oi) {
+                      const double2 *pf, const double2 *tw, double2 *acc, const int *oi) {
   const bool bastin = formula == LINQT_KUBO_BASTIN;
 #define LQ_FFT(r3) \
   bastin ? launch_fft<r3, 8>(s, L, Rv, nsites, M, pf, acc, oi) : launch_fft<r3, 4>(s, L, Rv, nsites, M, pf, acc, oi)
@@ -569,9 +565,9 @@ void kubo_fft_sites_t(Session *s, const Tin *L, const Tin *Rv, long nsites, int 
   }
 #undef LQ_FFT
   if (bastin)
-    launch_dft<8>(s, L, Rv, nsites, M, nump, pf, acc, oi);
+    launch_dft<8>(s, L, Rv, nsites, M, nump, pf, tw, acc, oi);
   else
-    launch_dft<4>(s, L, Rv, nsites, M, nump, pf, acc, oi);
+    launch_dft<4>(s, L, Rv, nsites, M, nump, pf, tw, acc, oi);
 }
 
 }  // namespace
@@ -586,19 +582,17 @@ double kubo_sites_us(long nsites, int M, int nump, int formula) {
   return 20 + nsites * (double)nump * M * seqs * 5.1e-7;
 }
 
-void kubo_prefactors(Session *s, int M, int nump, double2 *pf) {
-  k_prefactors<<<(M + 255) / 256, 256, 0, s->stream>>>(M, nump, pf);
-  LQ_LAUNCHED();
-}
-
 void kubo_fft_sites(Session *s, const void *Lv, const void *Rvv, long nsites, int M, int nump, int formula,
                     bool fp32_inputs, double2 *acc, const int *only_if) {
   double2 *pf = (double2 *)s->get("kubo_pf", sizeof(double2) * M);
-  kubo_prefactors(s, M, nump, pf);
+  const bool fft = shared_memory_fft(nump, formula);
+  double2 *tw = fft ? nullptr : (double2 *)s->get("kubo_tw", sizeof(double2) * nump);
+  k_prefactors<<<(std::max(M, fft ? 0 : nump) + 255) / 256, 256, 0, s->stream>>>(M, nump, pf, tw);
+  LQ_LAUNCHED();
   if (fp32_inputs)
-    kubo_fft_sites_t(s, (const float2 *)Lv, (const float2 *)Rvv, nsites, M, nump, formula, pf, acc, only_if);
+    kubo_fft_sites_t(s, (const float2 *)Lv, (const float2 *)Rvv, nsites, M, nump, formula, pf, tw, acc, only_if);
   else
-    kubo_fft_sites_t(s, (const double2 *)Lv, (const double2 *)Rvv, nsites, M, nump, formula, pf, acc, only_if);
+    kubo_fft_sites_t(s, (const double2 *)Lv, (const double2 *)Rvv, nsites, M, nump, formula, pf, tw, acc, only_if);
 }
 
 void kubo_postprocess(Session *s, const double2 *acc, int R, int nump, int formula, int N, double band_width,

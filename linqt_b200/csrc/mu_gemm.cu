@@ -169,13 +169,13 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
 }
 
 // Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo.  Where it is
-// rejected, raw += the FP64 product, by the grid of k_zgemm_cn_f64 (the last CTA of a tile adds its
-// parts, in order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that
-// the usual one costs 5 us and no host decision.
+// rejected, raw += the FP64 product in S slices of K (the last CTA of a tile adds its parts, in
+// order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that the usual one
+// costs a few us and no host decision.
 __global__ void __launch_bounds__(256, 2)
     k_commit(RnsStats *stats, RnsSide *side, int nchunk, const double2 *__restrict__ hi,
              const double2 *__restrict__ lo, const double2 *__restrict__ L, const double2 *__restrict__ Rv, int M, long K,
-             long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
+             unsigned S, long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
              double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo) {
   __shared__ bool last;
   const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)));
@@ -195,12 +195,12 @@ __global__ void __launch_bounds__(256, 2)
         tab_lo[t] = make_double2(re.y, im.y);
       }
     }
-  } else if (raw) {
+  } else if (raw && blockIdx.z < S) {
     zgemm_block(L, Rv, M, M, K, kchunk, part);
     unsigned *count = tiles + blockIdx.y * gridDim.x + blockIdx.x;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.z - 1;
+    if (threadIdx.x == 0) last = atomicAdd(count, 1u) == S - 1;
     __syncthreads();
     if (last) {
       __threadfence();
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256, 2)
         if (i >= M || j >= M) continue;
         const size_t t = (size_t)i * M + j;
         double2 s = raw[t];
-        for (unsigned z = 0; z < gridDim.z; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
+        for (unsigned z = 0; z < S; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
         raw[t] = s;
       }
       if (threadIdx.x == 0) *count = 0;
@@ -325,20 +325,10 @@ void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 
   LQ_LAUNCHED();
 }
 
-namespace {
-dim3 commit_grid(Session *s, int M, long K, bool moments, long *kchunk) {
-  const KSplit k = moments ? split_k(s, M, M, K) : KSplit{1, K};
-  *kchunk = k.kchunk;
-  return dim3((M + BN - 1) / BN, (M + BM - 1) / BM, (unsigned)k.S);
-}
-}  // namespace
-
 // The buffers of the FP64 kernel first: they are the ones that a solve cannot do without.
 int mu_reserve_rns(Session *s, int M, long K, bool moments) {
-  long kchunk = 0;
-  const dim3 grid = commit_grid(s, M, K, moments, &kchunk);
-  if (moments) s->get("zgemm_parts", sizeof(double2) * (size_t)grid.z * M * M);
-  s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
+  if (moments) s->get("zgemm_parts", sizeof(double2) * (size_t)split_k(s, M, M, K).S * M * M);
+  s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)((M + BM - 1) / BM) * ((M + BN - 1) / BN));
   return rns_reserve(s, M, M, K);
 }
 
@@ -346,15 +336,18 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
                            double2 *mu_raw, double2 *tab) {
   LQ_REQUIRE(!(fp32_inputs && mu_raw), "residues: moments of FP64 blocks only");
   const size_t MM = (size_t)M * M;
-  long kchunk = 0;
-  const dim3 grid = commit_grid(s, M, K, mu_raw != nullptr, &kchunk);
-  double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)grid.z * MM) : nullptr;
+  const KSplit k = split_k(s, M, M, K);
+  dim3 grid((M + BN - 1) / BN, (M + BM - 1) / BM);
+  // a pass of a CTA over its entries is one round trip: one pass where the tiles do not fill the device
+  grid.z = std::max(1, std::min(BM * BN / 256, s->sm_count * 4 / (int)(grid.x * grid.y)));
+  if (mu_raw) grid.z = std::max(grid.z, (unsigned)k.S);
+  double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MM) : nullptr;
   unsigned *tiles = (unsigned *)s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
   const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
   const size_t smem = zgemm_smem(sizeof(double2));
   raise_smem_limit((const void *)k_commit, smem);
   k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
-                                           M, K, kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr);
+                                           M, K, (unsigned)k.S, k.kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr);
   LQ_LAUNCHED();
   return &j.stats->rejected;
 }

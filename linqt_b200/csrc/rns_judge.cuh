@@ -32,40 +32,27 @@ __device__ __forceinline__ void raise_to(unsigned long long *a, double v) {
 // Whether the sum may be off by more than kAccept of its largest value `top`.  A value of a row is
 // off by up to half its unit, as if at random, so a sum with the rows' units ua, ub and norms |a|,
 // |b| by (ua |b| (+) ub |a|) / sqrt(6), (+) and the chunks in quadrature; the largest of the rows
-// stand for all.  By one block; not finite: rejected.
-__device__ inline bool judge(const RnsSide *side, int nchunk, double top) {
-  __shared__ double red[256];
-  double big = 0.0, sum = 0.0;
-  for (int pass = 0; pass < 2; ++pass) {
-    for (int c = threadIdx.x; c < nchunk; c += blockDim.x) {
-      double u[2], n[2];
-      for (int z = 0; z < 2; ++z) {
-        const RnsSide &sd = side[2 * c + z];
-        double t = 0.0;
-        for (int p = 0; p < kMaxParts; ++p) t += __longlong_as_double((long long)__ldcg(&sd.sq[p]));
-        u[z] = __longlong_as_double((long long)__ldcg(&sd.unit));
-        n[z] = sqrt(t);
-      }
-      double x = u[0] * n[1], y = u[1] * n[0];
-      if (!(x < INFINITY && y < INFINITY)) x = y = INFINITY;
-      big = fmax(big, fmax(x, y));
-      if (pass) sum += (x / red[0]) * (x / red[0]) + (y / red[0]) * (y / red[0]);
+// stand for all.  By every warp for itself, the same in all; not finite: rejected.
+__device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double top) {
+  const double allowed = kAccept * top;
+  double sum = 0.0;
+  for (int c = threadIdx.x & 31; c < nchunk; c += 32) {
+    double u[2], n[2];
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+      const RnsSide &sd = side[2 * c + z];
+      double t = 0.0;
+#pragma unroll
+      for (int p = 0; p < kMaxParts; ++p) t += __longlong_as_double((long long)__ldcg(&sd.sq[p]));
+      u[z] = __longlong_as_double((long long)__ldcg(&sd.unit));
+      n[z] = sqrt(t);
     }
-    if (pass) {
-      big = red[0];
-      __syncthreads();
-    }
-    red[threadIdx.x] = pass ? sum : big;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o)
-        red[threadIdx.x] = pass ? red[threadIdx.x] + red[threadIdx.x + o] : fmax(red[threadIdx.x], red[threadIdx.x + o]);
-      __syncthreads();
-    }
-    if (pass == 0 && red[0] == 0.0) return false;  // a side is zero
-    if (pass == 0 && red[0] == INFINITY) return true;
+    const double x = u[0] * n[1], y = u[1] * n[0];
+    if (x != 0.0) sum += (x / allowed) * (x / allowed);
+    if (y != 0.0) sum += (y / allowed) * (y / allowed);
   }
-  return !(big * sqrt(red[0] / 6.0) <= kAccept * top);
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  return !(sum <= 6.0);
 }
 
 }  // namespace linqt
