@@ -173,12 +173,12 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
 // order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that the usual one
 // costs a few us and no host decision.
 __global__ void __launch_bounds__(256, 2)
-    k_commit(RnsStats *stats, RnsSide *side, int nchunk, const double2 *__restrict__ hi,
+    k_commit(RnsStats *stats, RnsSide *side, int nchunk, double accept, const double2 *__restrict__ hi,
              const double2 *__restrict__ lo, const double2 *__restrict__ L, const double2 *__restrict__ Rv, int M, long K,
              unsigned S, long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
              double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo) {
   __shared__ bool last;
-  const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)));
+  const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)), accept);
   const int m0 = blockIdx.y * BM, m1 = blockIdx.x * BN;
   if (!no) {
     for (int e = threadIdx.x + 256 * blockIdx.z; e < BM * BN; e += 256 * gridDim.z) {
@@ -346,7 +346,7 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
   const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
   const size_t smem = zgemm_smem(sizeof(double2));
   raise_smem_limit((const void *)k_commit, smem);
-  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
+  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, tab ? kAcceptSigma : kAcceptMoments, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
                                            M, K, (unsigned)k.S, k.kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr);
   LQ_LAUNCHED();
   return &j.stats->rejected;

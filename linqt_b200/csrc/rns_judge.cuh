@@ -20,21 +20,23 @@ struct RnsStats {
   unsigned done;                       // blocks of k_commit
   int rejected;
 };
-// The error allowed, of the sum's largest value: 8 units of FP64 rounding.  The estimate for random
-// states is a tenth of it and less, and at most about one unit in a table that is noise alone
-// (operators whose products average out).
-constexpr double kAccept = 8.8817841970012523e-16;  // 2^-50
+// The error allowed, of the sum's largest value.  Moments: 8 units of FP64 rounding.  Tables for sigma: one,
+// since the Bastin integrand multiplies a table's errors by 1e6 (1024 energies, band edge) and the
+// bar of 1e-10 is that of a table rounded to FP64.  The estimate for random states is 5 / sqrt(K)
+// units, and about one in a table that is noise alone (operators whose products average out).
+constexpr double kAcceptMoments = 8.8817841970012523e-16;  // 2^-50
+constexpr double kAcceptSigma = 1.1102230246251565e-16;    // 2^-53
 
 __device__ __forceinline__ void raise_to(unsigned long long *a, double v) {
   atomicMax(a, (unsigned long long)__double_as_longlong(v));
 }
 
-// Whether the sum may be off by more than kAccept of its largest value `top`.  A value of a row is
+// Whether the sum may be off by more than `accept` of its largest value `top`.  A value of a row is
 // off by up to half its unit, as if at random, so a sum with the rows' units ua, ub and norms |a|,
 // |b| by (ua |b| (+) ub |a|) / sqrt(6), (+) and the chunks in quadrature; the largest of the rows
 // stand for all.  By every warp for itself, the same in all; not finite: rejected.
-__device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double top) {
-  const double allowed = kAccept * top;
+__device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double top, double accept) {
+  const double allowed = accept * top;
   double sum = 0.0;
   for (int c = threadIdx.x & 31; c < nchunk; c += 32) {
     double u[2], n[2];
@@ -52,7 +54,7 @@ __device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double to
     if (y != 0.0) sum += (y / allowed) * (y / allowed);
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  return !(sum <= 6.0);
+  return !(sum <= 6.0 && top < INFINITY);
 }
 
 }  // namespace linqt

@@ -99,3 +99,14 @@ def test_fp32_conductivity_of_regions_apart(oracle_lib):
                                                           0.0)[2][inner], chain(N, W), 2.0 ** -24)
     assert 10 * last_bits < np.abs(want).max()
     assert np.abs(integ[inner] - want).max() <= 10 * last_bits
+
+
+def test_sums_beyond_the_range_are_those_of_fp64_products(oracle_lib):
+    """States of 1e155: products overflow, and come out infinite or NaN, not as some finite sum."""
+    N, M = 600, 170
+    (H, V), _ = operators(oracle_lib, chain(N, 1.0), current(N, 0, N))
+    st = lattices.random_phase_states(N, 1, seed=3)
+    ok = lq.moments2d(H, V, V, st, M)
+    mu = lq.moments2d(H, V, V, st * 1e156, M)
+    large = np.abs(ok) > 1e-3 * np.abs(ok).max()
+    assert not np.isfinite(mu[large]).any()
