@@ -996,7 +996,6 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
   char *Rs = (char *)s->get("lr_R", blk * M);
   char *tmp = (char *)s->get("lr_tmp", blk * 4);
   double2 *raw = (double2 *)s->get("mu_raw", sizeof(double2) * (size_t)M * M);
-  LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * (size_t)M * M, s->stream));
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
     {
@@ -1006,7 +1005,7 @@ static void moments2d_dev(Session *s, const DeviceOp &H, const DeviceOp *opl, co
     }
     {
       PhaseScope ph(s, PH_CONTRACT);
-      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw);
+      mu_contract(s, Ls, Rs, M, (long)N * ch.Rc, fp32, o.precision, raw, c == 0);
       ph.launches(2);
     }
   }
@@ -1066,10 +1065,7 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     ~TableUse() { s->table_in_use = false; }
   } table_use{s};
   const size_t MM = (size_t)M * M;
-  if (mu) {
-    raw = (double2 *)s->get("mu_raw", sizeof(double2) * MM);
-    LQ_CUDA(cudaMemsetAsync(raw, 0, sizeof(double2) * MM, s->stream));
-  }
+  if (mu) raw = (double2 *)s->get("mu_raw", sizeof(double2) * MM);
   // sigma's site sums: from the raw table in double-double (kubo_table.cu), once per solve, or from
   // the transforms of every site (kubo_fft.cu), by the times both take at these sizes; the FP64
   // moments need the same table, so there only what the residues cost beyond the FP64 kernel
@@ -1086,10 +1082,10 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
     LQ_CUDA(cudaMemsetAsync(acc, 0, sizeof(double2) * 2 * (size_t)nump, s->stream));
     if (s->rns_budget &&
         kubo_table_us(M, nump, formula) + ch.nchunks * extra_us < ch.nchunks * kubo_sites_us(K, M, nump, formula))
-      tab = kubo_table_reserve(s, M, nump);
+      tab = kubo_table_reserve(s, M, nump, formula);
     s->table_in_use = tab != nullptr;
-    if (tab) LQ_CUDA(cudaMemsetAsync(tab, 0, sizeof(double2) * 2 * MM, s->stream));
   }
+  bool tab_empty = true;  // nothing in the table yet
   for (int c = 0; c < ch.nchunks; ++c) {
     void *phi = tmp + 3 * blk;
     {
@@ -1104,16 +1100,17 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
       PhaseScope ph(s, PH_CONTRACT);
       if (tab && !fp32) slab = mu_reserve_rns(s, M, K, true);
       if (slab)
-        rejected = mu_contract_rns(s, Ls, Rs, M, K, false, slab, raw, tab);
+        rejected = mu_contract_rns(s, Ls, Rs, M, K, false, slab, raw, c == 0, tab, tab_empty);
       else
-        mu_contract(s, Ls, Rs, M, K, fp32, o.precision, raw);
+        mu_contract(s, Ls, Rs, M, K, fp32, o.precision, raw, c == 0);
       ph.launches(2);
     }
     if (out) {
       PhaseScope ph(s, PH_FFT);
       if (tab && !(mu && !fp32)) slab = mu_reserve_rns(s, M, K, false);
       if (slab) {
-        if (!rejected) rejected = mu_contract_rns(s, Ls, Rs, M, K, fp32, slab, nullptr, tab);
+        if (!rejected) rejected = mu_contract_rns(s, Ls, Rs, M, K, fp32, slab, nullptr, false, tab, tab_empty);
+        tab_empty = false;
         kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc, rejected);
       } else {
         kubo_fft_sites(s, Ls, Rs, K, M, nump, formula, fp32, acc_c);
@@ -1122,7 +1119,7 @@ static void kubo_solve(Session *s, const DeviceOp &H, const DeviceOp *opl, const
       ph.launches(4);
     }
   }
-  if (tab) {
+  if (!tab_empty) {
     PhaseScope ph(s, PH_FFT);
     kubo_table_sums(s, tab, tab + MM, M, nump, formula, acc);
     ph.launches(5);

@@ -350,14 +350,14 @@ void moments1d_from_dots(Session *s, const double2 *dots, int steps, int M, int 
 // C(i,j) (+)= sum_k conj(A[i][k]) B[j][k], FP64
 void zgemm_cn(Session *s, const double2 *A, int MA, const double2 *B, int MB, long K, double2 *C, bool accumulate);
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw);
+                 double2 *mu_raw, bool first);
 // The same from the residues (mu_rns.cu), and the table in double-double into tab [2][M][M] (hi, lo);
-// mu_raw (FP64 blocks) or tab may be NULL.  Returns the device's judgement: where it is 1, the residues'
+// mu_raw (FP64 blocks) or tab may be NULL.  first: it holds nothing yet (else it is added to).  Returns the device's judgement: where it is 1, the residues'
 // rounding could have moved the table, mu_raw got the FP64 kernel's sum and tab nothing.  `slab` is
 // what mu_reserve_rns gave just before: not 0.
 int mu_reserve_rns(Session *s, int M, long K, bool moments);
 const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int slab,
-                           double2 *mu_raw, double2 *tab);
+                           double2 *mu_raw, bool raw_first, double2 *tab, bool tab_first);
 // Contraction in residues on the INT8 tensor cores, exact up to the rounding of its inputs
 // to a common exponent (mu_rns.cu).  rns_faster: whether an FP64 product is faster there; rns_us: its time;
 // rns_reserve: the chunks of K at a time whose buffers it holds (0: memory is short, use the FP64
@@ -406,13 +406,13 @@ inline size_t i8_digit_bytes(int digits, int M, long K) {
 
 // FFT path: accumulate p/w over all sites into acc[2*nump] (complex)
 // prefactors pf_m of Kubo_solver_FFT (kubo_fft.cu)
-// only_if: acc += them, on the device where *only_if is set
+// only_if: acc += them, on the device where *only_if is set (weights of kubo_table_reserve)
 void kubo_fft_sites(Session *s, const void *L, const void *Rv, long nsites, int M, int nump, int formula,
                     bool fp32_inputs, double2 *acc, const int *only_if = nullptr);
 // acc += the same from the raw moment table hi + lo (kubo_table.cu); its time, and that of the site
 // transforms of one call (us)
 // (kubo_table_reserve: whether its buffers are held, the table [2][M][M] among them)
-double2 *kubo_table_reserve(Session *s, int M, int nump);
+double2 *kubo_table_reserve(Session *s, int M, int nump, int formula);
 void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, int nump, int formula, double2 *acc);
 double kubo_table_us(int M, int nump, int formula);
 double kubo_sites_us(long nsites, int M, int nump, int formula);

@@ -29,6 +29,7 @@
 #include <cmath>
 
 #include "internal.cuh"
+#include "kubo_sites.cuh"
 
 namespace linqt {
 
@@ -151,23 +152,10 @@ __device__ __forceinline__ void greenwood_product(const double2 *X, int stride, 
   p.x += rb.x * rk.x + ib.x * ik.x;
 }
 
-// prefactors pf_m (src/Bastin_FFTs.cpp:20-21, include/Kubo_solver_FFT.hpp:99-107), and for the direct
-// transforms the roots of unity tw
 __global__ void k_prefactors(int M, int nump, double2 *__restrict__ pf, double2 *__restrict__ tw) {
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    const double g = 1 / (M + 1.0) *
-                     ((M - m + 1.0) * cos(M_PI * m / (M + 1.0)) + sin(M_PI * m / (M + 1.0)) / tan(M_PI / (M + 1.0)));
-    const double amp = (2 - (m == 0)) * g;
-    double sn, cs;
-    sincos(M_PI * m / (2.0 * nump), &sn, &cs);
-    pf[m] = make_double2(amp * cs, amp * sn);
-  }
-  if (!tw) return;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nump; t += gridDim.x * blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * t / nump, &sn, &cs);
-    tw[t] = make_double2(cs, sn);
-  }
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+  for (int m = t0; m < M; m += st) pf[m] = site_prefactor(m, M, nump);
+  for (int t = t0; tw && t < nump; t += st) tw[t] = site_root(t, nump);
 }
 
 constexpr int kFftThreads = 512;
@@ -582,13 +570,19 @@ double kubo_sites_us(long nsites, int M, int nump, int formula) {
   return 20 + nsites * (double)nump * M * seqs * 5.1e-7;
 }
 
+SiteTables site_tables(Session *s, int M, int nump, int formula) {
+  return {(double2 *)s->get("kubo_pf", sizeof(double2) * (size_t)M),
+          shared_memory_fft(nump, formula) ? nullptr : (double2 *)s->get("kubo_tw", sizeof(double2) * (size_t)nump)};
+}
+
 void kubo_fft_sites(Session *s, const void *Lv, const void *Rvv, long nsites, int M, int nump, int formula,
                     bool fp32_inputs, double2 *acc, const int *only_if) {
-  double2 *pf = (double2 *)s->get("kubo_pf", sizeof(double2) * M);
-  const bool fft = shared_memory_fft(nump, formula);
-  double2 *tw = fft ? nullptr : (double2 *)s->get("kubo_tw", sizeof(double2) * nump);
-  k_prefactors<<<(std::max(M, fft ? 0 : nump) + 255) / 256, 256, 0, s->stream>>>(M, nump, pf, tw);
-  LQ_LAUNCHED();
+  const SiteTables t = site_tables(s, M, nump, formula);
+  double2 *pf = t.pf, *tw = t.tw;
+  if (!only_if) {
+    k_prefactors<<<(std::max(M, tw ? nump : 0) + 255) / 256, 256, 0, s->stream>>>(M, nump, pf, tw);
+    LQ_LAUNCHED();
+  }
   if (fp32_inputs)
     kubo_fft_sites_t(s, (const float2 *)Lv, (const float2 *)Rvv, nsites, M, nump, formula, pf, tw, acc, only_if);
   else

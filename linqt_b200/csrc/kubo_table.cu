@@ -26,14 +26,24 @@
 
 #include "dd.cuh"
 #include "internal.cuh"
+#include "kubo_sites.cuh"
 
 namespace linqt {
 
 namespace {
 
-// cos(pi q / (2 n)) for q < 4 n in double-double: Taylor series of sine and cosine on [0, pi/4]
-__global__ void k_dd_cosines(int n, double2 *__restrict__ tab) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < 4 * n; q += gridDim.x * blockDim.x) {
+// All that depends on the sizes alone, in one launch: cos(pi q / (2 n)) for q < 4 n in double-double
+// (Taylor series of sine and cosine on [0, pi/4]), the amplitudes, and the weights of the site
+// transforms, which take the blocks whose table is rejected.
+__global__ void k_table_setup(int n, int M, double2 *__restrict__ tab, double *__restrict__ amp,
+                              double2 *__restrict__ pf, double2 *__restrict__ tw) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, st = gridDim.x * blockDim.x;
+  for (int m = t0; m < M; m += st) {
+    amp[m] = site_amplitude(m, M);
+    pf[m] = site_prefactor(m, M, n);
+  }
+  for (int t = t0; tw && t < n; t += st) tw[t] = site_root(t, n);
+  for (int q = t0; q < 4 * n; q += st) {
     const int quad = q / n;
     int r = q % n;
     const bool swap = 2 * r > n;  // use the complement
@@ -55,17 +65,6 @@ __global__ void k_dd_cosines(int n, double2 *__restrict__ tab) {
     }
     tab[q] = quad == 0 ? c : quad == 1 ? dd_neg(s) : quad == 2 ? dd_neg(c) : s;
   }
-}
-
-// a_m (include/Kubo_solver_FFT.hpp:99-107), as k_prefactors of kubo_fft.cu forms it
-__device__ __forceinline__ double amplitude(int m, int M) {
-  const double g = 1 / (M + 1.0) *
-                   ((M - m + 1.0) * cos(M_PI * m / (M + 1.0)) + sin(M_PI * m / (M + 1.0)) / tan(M_PI / (M + 1.0)));
-  return (2 - (m == 0)) * g;
-}
-
-__global__ void k_amplitudes(int M, double *__restrict__ amp) {
-  for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) amp[m] = amplitude(m, M);
 }
 
 // h(m, m') = a_m' U_s(m, m') as two dd numbers (re, im)
@@ -261,11 +260,15 @@ TableBuffers table_buffers(Session *s, int M, int n) {
 }
 }  // namespace
 
-// The raw table's buffer, with all that kubo_table_sums needs beside it; NULL where memory is short (the
-// site transforms do without them).
-double2 *kubo_table_reserve(Session *s, int M, int nump) {
+// The raw table's buffer, with all that kubo_table_sums needs beside it, its weights and those of the site
+// transforms formed; NULL where memory is short (the site transforms do without).
+double2 *kubo_table_reserve(Session *s, int M, int nump, int formula) {
+  const SiteTables t = site_tables(s, M, nump, formula);
   try {
-    return table_buffers(s, M, nump).table;
+    const TableBuffers b = table_buffers(s, M, nump);
+    k_table_setup<<<(std::max(M, 4 * nump) + 127) / 128, 128, 0, s->stream>>>(nump, M, b.cosines, b.amp, t.pf, t.tw);
+    LQ_LAUNCHED();
+    return b.table;
   } catch (const Error &e) {
     if (e.code != LINQT_ERR_NOMEM || s->strict_memory) throw;
     s->release("kt_");
@@ -282,10 +285,6 @@ void kubo_table_sums(Session *s, const double2 *hi, const double2 *lo, int M, in
   const TableBuffers b = table_buffers(s, M, n);
   double2 *tab = b.cosines, *re = b.coef, *im = re + (size_t)M * M, *part = b.part;
   double *amp = b.amp;
-  k_dd_cosines<<<(4 * n + 127) / 128, 128, 0, s->stream>>>(n, tab);
-  LQ_LAUNCHED();
-  k_amplitudes<<<(M + 127) / 128, 128, 0, s->stream>>>(M, amp);
-  LQ_LAUNCHED();
   const long tot = (long)M * M;
   const int g = (int)std::max(1L, std::min((tot + 255) / 256, (long)s->sm_count * 8));
   k_table_coef<<<g, 256, 0, s->stream>>>(hi, lo, amp, M, re, im);

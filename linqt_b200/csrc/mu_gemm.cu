@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
   zgemm_block(L, Rv, MA, MB, K, kchunk, part);
 }
 
-// Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo.  Where it is
+// Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo (first: =).  Where it is
 // rejected, raw += the FP64 product in S slices of K (the last CTA of a tile adds its parts, in
 // order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that the usual one
 // costs a few us and no host decision.
@@ -176,26 +176,28 @@ __global__ void __launch_bounds__(256, 2)
     k_commit(RnsStats *stats, RnsSide *side, int nchunk, double accept, const double2 *__restrict__ hi,
              const double2 *__restrict__ lo, const double2 *__restrict__ L, const double2 *__restrict__ Rv, int M, long K,
              unsigned S, long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
-             double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo) {
+             double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo, bool raw_first, bool tab_first) {
   __shared__ bool last;
+  const double2 zero = make_double2(0.0, 0.0);
   const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)), accept);
   const int m0 = blockIdx.y * BM, m1 = blockIdx.x * BN;
-  if (!no) {
+  if (!no || (tab_first && tab_hi)) {
     for (int e = threadIdx.x + 256 * blockIdx.z; e < BM * BN; e += 256 * gridDim.z) {
       const int i = m0 + e / BN, j = m1 + e % BN;
       if (i >= M || j >= M) continue;
       const size_t t = (size_t)i * M + j;
-      const double2 h = hi[t];
-      if (raw) raw[t] = cadd(raw[t], h);
+      const double2 h = no ? zero : hi[t];
+      if (raw && !no) raw[t] = raw_first ? h : cadd(raw[t], h);
       if (tab_hi) {
-        const double2 l = lo[t], th = tab_hi[t], tl = tab_lo[t];
+        const double2 l = no ? zero : lo[t], th = tab_first ? zero : tab_hi[t], tl = tab_first ? zero : tab_lo[t];
         const double2 re = dd_add(make_double2(th.x, tl.x), make_double2(h.x, l.x));
         const double2 im = dd_add(make_double2(th.y, tl.y), make_double2(h.y, l.y));
         tab_hi[t] = make_double2(re.x, im.x);
         tab_lo[t] = make_double2(re.y, im.y);
       }
     }
-  } else if (raw && blockIdx.z < S) {
+  }
+  if (no && raw && blockIdx.z < S) {
     zgemm_block(L, Rv, M, M, K, kchunk, part);
     unsigned *count = tiles + blockIdx.y * gridDim.x + blockIdx.x;
     __threadfence();
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(256, 2)
         const int i = m0 + e / BN, j = m1 + e % BN;
         if (i >= M || j >= M) continue;
         const size_t t = (size_t)i * M + j;
-        double2 s = raw[t];
+        double2 s = raw_first ? zero : raw[t];
         for (unsigned z = 0; z < S; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
         raw[t] = s;
       }
@@ -333,7 +335,7 @@ int mu_reserve_rns(Session *s, int M, long K, bool moments) {
 }
 
 const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int slab,
-                           double2 *mu_raw, double2 *tab) {
+                           double2 *mu_raw, bool raw_first, double2 *tab, bool tab_first) {
   LQ_REQUIRE(!(fp32_inputs && mu_raw), "residues: moments of FP64 blocks only");
   const size_t MM = (size_t)M * M;
   const KSplit k = split_k(s, M, M, K);
@@ -347,17 +349,19 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
   const size_t smem = zgemm_smem(sizeof(double2));
   raise_smem_limit((const void *)k_commit, smem);
   k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, tab ? kAcceptSigma : kAcceptMoments, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
-                                           M, K, (unsigned)k.S, k.kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr);
+                                           M, K, (unsigned)k.S, k.kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr,
+                                           raw_first, tab_first);
   LQ_LAUNCHED();
   return &j.stats->rejected;
 }
 
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
-                 double2 *mu_raw) {
+                 double2 *mu_raw, bool first) {
+  const int slab = !fp32_inputs && rns_faster(M, M, K) ? mu_reserve_rns(s, M, K, true) : 0;
+  if (first && !slab) LQ_CUDA(cudaMemsetAsync(mu_raw, 0, sizeof(double2) * (size_t)M * M, s->stream));
   if (!fp32_inputs) {
-    const int slab = rns_faster(M, M, K) ? mu_reserve_rns(s, M, K, true) : 0;
     if (slab)
-      (void)mu_contract_rns(s, L, Rv, M, K, false, slab, mu_raw, nullptr);
+      (void)mu_contract_rns(s, L, Rv, M, K, false, slab, mu_raw, first, nullptr, false);
     else
       zgemm_cn_t<double2>(s, (const double2 *)L, M, (const double2 *)Rv, M, K, mu_raw, true);
   } else if (i8_digits(precision)) {
