@@ -51,10 +51,14 @@ enum {
 enum { LINQT_STORAGE_HERMITIAN_UPPER = 0, LINQT_STORAGE_GENERAL = 1 };
 
 enum {
-  LINQT_PREC_FP64 = 0,       /* FP64 recursion, FP64 moment contraction */
+  LINQT_PREC_FP64 = 0,       /* FP64 recursion; FP64 moment contraction, of large tables in residues on the
+                                INT8 tensor cores where their rounding cannot reach 8 FP64 units of the
+                                table's maximum */
   LINQT_PREC_MIXED = 1,      /* FP32 Chebyshev vectors (FP64 operators and accumulation in the recursion),
                                 moment contraction on the INT8 tensor cores from 4-digit (28-bit) splits
-                                of the FP32 blocks with exact INT32 accumulation, FP64 across chunks */
+                                of the FP32 blocks with exact INT32 accumulation, FP64 across chunks.  Faster
+                                than LINQT_PREC_FP64 for moments; a whole Kubo-Bastin solve contracts twice
+                                (digits for the moments, residues for sigma) and may be slower than in FP64 */
   LINQT_PREC_FP32 = 2,       /* FP32 vectors, FP64 MMA contraction of the FP32 blocks (diagnostic) */
   LINQT_PREC_MIXED_TF32 = 3, /* FP32 vectors, 3xTF32 tensor-core contraction with FP32 accumulation over
                                 2048-float chunks (the split-precision form; its truncating FP32

@@ -6,8 +6,9 @@
 // a barrier costs the stores' acknowledgement, the addition's way to L2 and one poll, about
 // 1 us; a last arrival that resets a count and bumps a generation adds two dependent round
 // trips, and sleeping between polls half of a poll (a recursion step of 961 rows on 4 CTAs took
-// 4.4 us with these and takes 2.3 us; of 65536 rows on 256 CTAs, 4.5 and 2.4 us).  Arrival and wait are separate, so that work
-// whose results no other CTA reads in the next step (the dot products) runs between them.
+// 4.4 us with these and takes 2.3 us; of 65536 rows on 256 CTAs, 4.5 and 2.4 us).
+// Arrival and wait are separate, so that work whose results no other CTA reads in the next step
+// (the dot products) runs between them.
 //
 // The wait is bounded: after kSpinLimit polls a CTA sets the error flag and every waiting CTA
 // gives up, so a bad launch ends instead of hanging the GPU; the host turns the flag into
@@ -27,13 +28,14 @@ namespace linqt {
 
 struct GridBarrier {
   unsigned count;  // arrivals since the launch
-  unsigned unused;
   int err;
   int extra;              // fault injection (tests): arrivals awaited beyond the launched CTAs
   long long spin_limit;   // fault injection (tests): polls before giving up (0: kSpinLimit)
 };
 // bytes of GridBarrier that restart at zero for every launch
 constexpr size_t kBarrierResetBytes = offsetof(GridBarrier, err);
+
+constexpr unsigned kFewCtas = 2 * 148;  // two CTAs on each of a B200's SMs
 
 constexpr long long kSpinLimit = 1LL << 24;  // polls of a few 0.1 us: well above any step, far below a hang
 
@@ -88,7 +90,7 @@ __device__ __forceinline__ bool grid_wait(GridBarrier *bar) {
     // An acquire drops the SM's L1 lines.  Up to two CTAs an SM (256 CTAs: 0.4 us less a
     // barrier than a fence after the poll) every poll is one; with more, whose other CTAs
     // would read on through a cold L1 meanwhile, only the last load is.
-    const bool few = st.need <= 296;
+    const bool few = st.need <= kFewCtas;
     for (long long spins = 1;; ++spins) {
       const unsigned c = few ? load_acquire(&bar->count) : load_relaxed(&bar->count);
       if ((int)(c - target) >= 0) break;

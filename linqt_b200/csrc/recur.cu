@@ -16,9 +16,9 @@
 // afterwards in a fixed order.
 //
 // Vectors written in one step are read by other CTAs in the next.  The grid barrier
-// orders those writes before the next step's reads (release: bar.sync, fence, atomic;
-// acquire: poll, fence, bar.sync) and its gpu-scope fence invalidates stale L1 lines, so
-// vector loads may go through L1 (ld.global.ca), where a row's neighbours read by nearby
+// orders those writes before the next step's reads (release: bar.sync, then an addition with
+// release semantics; acquire: polls with acquire semantics, then bar.sync), and its acquire
+// drops stale L1 lines, so vector loads may go through L1 (ld.global.ca), where a row's neighbours read by nearby
 // rows of the same CTA hit.  Operators (read-only for the whole launch) use the
 // read-only path.  The operators are FP64 for either vector precision: FP32 blocks are
 // accumulated in FP64 and rounded once per entry and step.
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_1d<T>(VPT))
 #pragma unroll
       for (int u = 0; u < VPT; ++u) acc[u] = make_double2(0, 0);
       const size_t base = (size_t)row * ldx + coff + c0;
-      // The row's own T_{s-1}, T_s and (mode 1) phi.  One or two columns per thread: loaded
+      // The row's own T_{s-1}, T_s and (mode 1) phi.  Up to kHoist columns per thread: loaded
       // before the gathers, one L2 latency for all.  More columns would hold too many
       // registers meanwhile: only asked for in L2, and loaded after the gathers.
       C pv[VPT], xv[VPT], fv[VPT];
@@ -919,7 +919,7 @@ void dispatch(int R, int shape, Args &&...args) {
 
 }  // namespace
 
-// The barrier's count/generation restart at zero for every launch; its error flag is
+// The barrier's count restarts at zero for every launch; its error flag is
 // sticky until check_device_errors reads it.
 GridBarrier *barrier_for(Session *s) {
   Barrier *bar = (Barrier *)s->get("rec_barrier", sizeof(Barrier));
