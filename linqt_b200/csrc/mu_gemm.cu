@@ -171,15 +171,22 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
 // Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo (first: =).  Where it is
 // rejected, raw += the FP64 product in S slices of K (the last CTA of a tile adds its parts, in
 // order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that the usual one
-// costs a few us and no host decision.
-__global__ void __launch_bounds__(256, 2)
+// costs a few us and no host decision.  RAW false: without the product's registers and shared
+// memory, which leave two CTAs an SM (Greenwood, 300 moments: 19 us cold with them).
+template <bool RAW>
+__global__ void __launch_bounds__(256, RAW ? 2 : 4)
     k_commit(RnsStats *stats, RnsSide *side, int nchunk, double accept, const double2 *__restrict__ hi,
              const double2 *__restrict__ lo, const double2 *__restrict__ L, const double2 *__restrict__ Rv, int M, long K,
              unsigned S, long kchunk, double2 *__restrict__ part, unsigned *__restrict__ tiles, double2 *__restrict__ raw,
              double2 *__restrict__ tab_hi, double2 *__restrict__ tab_lo, bool raw_first, bool tab_first) {
-  __shared__ bool last;
+  __shared__ bool last, rejected;
   const double2 zero = make_double2(0.0, 0.0);
-  const bool no = judge(side, nchunk, __longlong_as_double((long long)__ldcg(&stats->top)), accept);
+  if (threadIdx.x < 32) {
+    const bool r = judge(side, nchunk, __longlong_as_double((long long)stats->top), accept);
+    if (threadIdx.x == 0) rejected = r;
+  }
+  __syncthreads();
+  const bool no = rejected;
   const int m0 = blockIdx.y * BM, m1 = blockIdx.x * BN;
   if (!no || (tab_first && tab_hi)) {
     for (int e = threadIdx.x + 256 * blockIdx.z; e < BM * BN; e += 256 * gridDim.z) {
@@ -187,7 +194,7 @@ __global__ void __launch_bounds__(256, 2)
       if (i >= M || j >= M) continue;
       const size_t t = (size_t)i * M + j;
       const double2 h = no ? zero : hi[t];
-      if (raw && !no) raw[t] = raw_first ? h : cadd(raw[t], h);
+      if (RAW && !no) raw[t] = raw_first ? h : cadd(raw[t], h);
       if (tab_hi) {
         const double2 l = no ? zero : lo[t], th = tab_first ? zero : tab_hi[t], tl = tab_first ? zero : tab_lo[t];
         const double2 re = dd_add(make_double2(th.x, tl.x), make_double2(h.x, l.x));
@@ -197,24 +204,26 @@ __global__ void __launch_bounds__(256, 2)
       }
     }
   }
-  if (no && raw && blockIdx.z < S) {
-    zgemm_block(L, Rv, M, M, K, kchunk, part);
-    unsigned *count = tiles + blockIdx.y * gridDim.x + blockIdx.x;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(count, 1u) == S - 1;
-    __syncthreads();
-    if (last) {
+  if constexpr (RAW) {
+    if (no && blockIdx.z < S) {
+      zgemm_block(L, Rv, M, M, K, kchunk, part);
+      unsigned *count = tiles + blockIdx.y * gridDim.x + blockIdx.x;
       __threadfence();
-      for (int e = threadIdx.x; e < BM * BN; e += 256) {
-        const int i = m0 + e / BN, j = m1 + e % BN;
-        if (i >= M || j >= M) continue;
-        const size_t t = (size_t)i * M + j;
-        double2 s = raw_first ? zero : raw[t];
-        for (unsigned z = 0; z < S; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
-        raw[t] = s;
+      __syncthreads();
+      if (threadIdx.x == 0) last = atomicAdd(count, 1u) == S - 1;
+      __syncthreads();
+      if (last) {
+        __threadfence();
+        for (int e = threadIdx.x; e < BM * BN; e += 256) {
+          const int i = m0 + e / BN, j = m1 + e % BN;
+          if (i >= M || j >= M) continue;
+          const size_t t = (size_t)i * M + j;
+          double2 s = raw_first ? zero : raw[t];
+          for (unsigned z = 0; z < S; ++z) s = cadd(s, __ldcg(part + (size_t)z * M * M + t));
+          raw[t] = s;
+        }
+        if (threadIdx.x == 0) *count = 0;
       }
-      if (threadIdx.x == 0) *count = 0;
     }
   }
   // every CTA has judged before the last one clears the statistics
@@ -341,14 +350,15 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
   const KSplit k = split_k(s, M, M, K);
   dim3 grid((M + BN - 1) / BN, (M + BM - 1) / BM);
   // a pass of a CTA over its entries is one round trip: one pass where the tiles do not fill the device
-  grid.z = std::max(1, std::min(BM * BN / 256, s->sm_count * 4 / (int)(grid.x * grid.y)));
+  grid.z = std::max(1, std::min(BM * BN / 256, s->sm_count * (mu_raw ? 2 : 4) / (int)(grid.x * grid.y)));
   if (mu_raw) grid.z = std::max(grid.z, (unsigned)k.S);
   double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MM) : nullptr;
   unsigned *tiles = (unsigned *)s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
   const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
-  const size_t smem = zgemm_smem(sizeof(double2));
-  raise_smem_limit((const void *)k_commit, smem);
-  k_commit<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, tab ? kAcceptSigma : kAcceptMoments, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
+  const size_t smem = mu_raw ? zgemm_smem(sizeof(double2)) : 0;
+  auto *f = mu_raw ? k_commit<true> : k_commit<false>;
+  raise_smem_limit((const void *)f, smem);
+  f<<<grid, 256, smem, s->stream>>>(j.stats, j.side, j.nchunk, tab ? kAcceptSigma : kAcceptMoments, j.hi, j.lo, (const double2 *)L, (const double2 *)Rv,
                                            M, K, (unsigned)k.S, k.kchunk, part, tiles, mu_raw, tab, tab ? tab + MM : nullptr,
                                            raw_first, tab_first);
   LQ_LAUNCHED();

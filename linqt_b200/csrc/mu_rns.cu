@@ -559,8 +559,13 @@ __global__ void __launch_bounds__(256)
                        (unsigned long long)__double_as_longlong(fabs(im.x))));
   }
   if (!last) return;
+  __shared__ unsigned long long top_s;
+  if (threadIdx.x == 0) top_s = 0;
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(&stats->top, top);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicMax(&top_s, top);
+  __syncthreads();
+  if (threadIdx.x == 0 && top_s > __ldcg(&stats->top)) atomicMax(&stats->top, top_s);
 }
 
 // [blocks][rows][128 bytes], box 128 bytes x 128 rows; rows past the end read as zero

@@ -34,7 +34,8 @@ __device__ __forceinline__ void raise_to(unsigned long long *a, double v) {
 // Whether the sum may be off by more than `accept` of its largest value `top`.  A value of a row is
 // off by up to half its unit, as if at random, so a sum with the rows' units ua, ub and norms |a|,
 // |b| by (ua |b| (+) ub |a|) / sqrt(6), (+) and the chunks in quadrature; the largest of the rows
-// stand for all.  By every warp for itself, the same in all; not finite: rejected.
+// stand for all.  By one warp of a CTA, through L1: with every warp of a few hundred CTAs reading these few
+// lines from L2, their one slice took 10 to 20 us.  Not finite: rejected.
 __device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double top, double accept) {
   const double allowed = accept * top;
   double sum = 0.0;
@@ -45,8 +46,8 @@ __device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double to
       const RnsSide &sd = side[2 * c + z];
       double t = 0.0;
 #pragma unroll
-      for (int p = 0; p < kMaxParts; ++p) t += __longlong_as_double((long long)__ldcg(&sd.sq[p]));
-      u[z] = __longlong_as_double((long long)__ldcg(&sd.unit));
+      for (int p = 0; p < kMaxParts; ++p) t += __longlong_as_double((long long)sd.sq[p]);
+      u[z] = __longlong_as_double((long long)sd.unit);
       n[z] = sqrt(t);
     }
     const double x = u[0] * n[1], y = u[1] * n[0];
