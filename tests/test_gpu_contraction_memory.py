@@ -94,6 +94,14 @@ def test_planes_left_behind_do_not_narrow_the_next_solve(solve, wanted, session)
 
 
 @pytest.mark.parametrize("sigma", [False, True])
+def test_one_chunk_of_planes_at_a_time_gives_the_same_bits(solve, wanted, session, sigma):
+    """Room for one of the four chunks' planes, and then for all."""
+    with only(int(6e9)):
+        assert np.array_equal(solve(session, sigma), wanted[sigma])
+    assert np.array_equal(solve(session, sigma), wanted[sigma])
+
+
+@pytest.mark.parametrize("sigma", [False, True])
 def test_no_size_of_the_rest_fails(solve, wanted, sigma):
     """The planes may take the rest of the memory, or nearly, but not what the solve needs besides."""
     n, ref = 2 * M * M, wanted[sigma]

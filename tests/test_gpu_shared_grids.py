@@ -30,3 +30,22 @@ def test_a_granted_share_is_the_whole_grid(ctas):
     got = srv.result(t).copy()
     srv.close()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("share", [0.02, 0.3, 0.7])
+@pytest.mark.parametrize("R", [1, 2])
+def test_a_share_too_small_for_the_registers(share, R):
+    """Blocks that the register recursion takes on the whole device, of a session whose share covers a part
+    of its grid: the other kernel's moments (the same terms in another order, below 1e-13)."""
+    N = 256 * 230 // R
+    i = np.arange(N)
+    H = lq.Operator.from_csr(N, *lattices.upper_csr(
+        N, np.concatenate([i] * 4), np.concatenate([(i + d) % N for d in range(4)]),
+        np.concatenate([0.2 * (lattices.uniform(5, N) - 0.5)] + [np.full(N, 0.13)] * 3)))
+    st = lattices.random_phase_states(N, R, seed=3)
+    want = lq.moments1d(H, None, st, 64)
+    s = lq.Session(0)
+    s.set_sm_share(share)
+    got = lq.moments1d(H, None, st, 64, session=s)
+    s.close()
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
