@@ -352,9 +352,9 @@ void zgemm_cn(Session *s, const double2 *A, int MA, const double2 *B, int MB, lo
 void mu_contract(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int precision,
                  double2 *mu_raw, bool first);
 // The same from the residues (mu_rns.cu), and the table in double-double into tab [2][M][M] (hi, lo);
-// mu_raw (FP64 blocks) or tab may be NULL.  first: it holds nothing yet (else it is added to).  Returns the device's judgement: where it is 1, the residues'
-// rounding could have moved the table, mu_raw got the FP64 kernel's sum and tab nothing.  `slab` is
-// what mu_reserve_rns gave just before: not 0.
+// mu_raw (FP64 blocks) or tab may be NULL.  first: it holds nothing yet (else it is added to).  Returns
+// a device flag: where it is 1, the residues' rounding could have moved the table, mu_raw got the
+// FP64 kernel's sum and tab nothing.  `slab` is what mu_reserve_rns gave just before: not 0.
 int mu_reserve_rns(Session *s, int M, long K, bool moments);
 const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, long K, bool fp32_inputs, int slab,
                            double2 *mu_raw, bool raw_first, double2 *tab, bool tab_first);
@@ -368,13 +368,13 @@ int rns_reserve(Session *s, int MA, int MB, long K);
 size_t rns_footprint(int MA, int MB, long K, size_t budget);
 struct RnsStats;
 struct RnsSide;
-struct RnsJudgement {
+struct RnsSum {
   const double2 *hi, *lo;  // the sum
   RnsStats *stats;
   RnsSide *side;
   int nchunk;
 };
-RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab);
+RnsSum zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab);
 void rns_clear_stats(Session *s);
 void mu_finalize(Session *s, const double2 *mu_raw, int M, int R, double2 *mu);
 void reduce_parts_into(Session *s, const double2 *part, int S, long MM, double2 *dst);

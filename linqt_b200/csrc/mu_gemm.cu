@@ -15,7 +15,7 @@
 // the long K axis with a fixed-order FP64 reduction (deterministic).
 #include "dd.cuh"
 #include "internal.cuh"
-#include "rns_judge.cuh"
+#include "rns_accept.cuh"
 
 namespace linqt {
 
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_cn_f64(const Tc *__restrict__ 
   zgemm_block(L, Rv, MA, MB, K, kchunk, part);
 }
 
-// Judges a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo (first: =).  Where it is
+// Checks a sum of the residues (mu_rns.cu) and commits it: raw += hi, tab += hi + lo (first: =).  Where it is
 // rejected, raw += the FP64 product in S slices of K (the last CTA of a tile adds its parts, in
 // order), and tab stays.  raw or tab may be NULL.  One launch for both outcomes, so that the usual one
 // costs a few us and no host decision.  RAW false: without the product's registers and shared
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256, RAW ? 2 : 4)
   __shared__ bool last, rejected;
   const double2 zero = make_double2(0.0, 0.0);
   if (threadIdx.x < 32) {
-    const bool r = judge(side, nchunk, __longlong_as_double((long long)stats->top), accept);
+    const bool r = rns_rejected(side, nchunk, __longlong_as_double((long long)stats->top), accept);
     if (threadIdx.x == 0) rejected = r;
   }
   __syncthreads();
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256, RAW ? 2 : 4)
       }
     }
   }
-  // every CTA has judged before the last one clears the statistics
+  // every CTA has checked before the last one clears the statistics
   __syncthreads();
   if (threadIdx.x == 0)
     last = atomicAdd(&stats->done, 1u) == gridDim.x * gridDim.y * gridDim.z - 1;
@@ -354,7 +354,7 @@ const int *mu_contract_rns(Session *s, const void *L, const void *Rv, int M, lon
   if (mu_raw) grid.z = std::max(grid.z, (unsigned)k.S);
   double2 *part = mu_raw ? (double2 *)s->get("zgemm_parts", sizeof(double2) * (size_t)k.S * MM) : nullptr;
   unsigned *tiles = (unsigned *)s->get("mu_tiles_counter", sizeof(unsigned) * (size_t)grid.x * grid.y);
-  const RnsJudgement j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
+  const RnsSum j = zgemm_cn_rns(s, L, M, Rv, M, K, fp32_inputs, slab);
   const size_t smem = mu_raw ? zgemm_smem(sizeof(double2)) : 0;
   auto *f = mu_raw ? k_commit<true> : k_commit<false>;
   raise_smem_limit((const void *)f, smem);

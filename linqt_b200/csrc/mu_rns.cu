@@ -20,7 +20,7 @@
 //     below half the product of the moduli), scaled back and added over the chunks in
 //     double-double arithmetic (k_rns_crt).  The sum comes as hi + lo, so that the energy
 //     reconstruction (kubo_table.cu) may use more than 53 bits of it.
-//  5. The sum is accepted or not, on the device (judge in rns_judge.cuh, k_commit in mu_gemm.cu).
+//  5. The sum is accepted or not, on the device (rns_rejected in rns_accept.cuh, k_commit in mu_gemm.cu).
 //
 // Against the FP64 tensor-core kernel (mu_gemm.cu), whose partial sums round once per term, the
 // only error is that of step 1, which averages over K: a value keeps the bits above 2^-53 of its
@@ -29,7 +29,7 @@
 // local state 1.4e-16; FP64 products 1.6e-16 and 3.5e-16).  Where one is large only where the other
 // is small, the table lives on the small values: currents in two regions that the states hardly
 // connect were off by 5e-11 of the maximum, or all of it (FP64 products 5e-16).  So step 1's error
-// is estimated from what it did, the rows' units and norms (rns_judge.cuh), and a sum that it could
+// is estimated from what it did, the rows' units and norms (rns_accept.cuh), and a sum that it could
 // move by more than is allowed there is dropped for the FP64 kernel's, and sigma's for the site
 // transforms.  That costs one launch and the rows' sums of squares: graphene 128 x 128, 8
 // vectors, 512 moments 5.75 -> 5.85 ms.
@@ -47,7 +47,7 @@
 
 #include "dd.cuh"
 #include "internal.cuh"
-#include "rns_judge.cuh"
+#include "rns_accept.cuh"
 #include "tc_common.cuh"
 
 namespace linqt {
@@ -655,7 +655,7 @@ int rns_reserve(Session *s, int MA, int MB, long K) {
   long want = slab_of(p, s->rns_budget);
   long held = std::min({(long)(held_bytes(s, "rns_planes") / p.planes), (long)(held_bytes(s, "rns_res") / p.res),
                         (long)(held_bytes(s, "rns_exp") / p.exps)});
-  if (held_bytes(s, "rns_sum") < sum || held_bytes(s, "mu_sides_counter") < sides || !held_bytes(s, "mu_judge_counter") ||
+  if (held_bytes(s, "rns_sum") < sum || held_bytes(s, "mu_sides_counter") < sides || !held_bytes(s, "mu_stats_counter") ||
       !held_bytes(s, "mu_tc_err_barrier"))
     held = 0;
   if (held >= want || s->capturing) return (int)std::min(held, want);
@@ -669,7 +669,7 @@ int rns_reserve(Session *s, int MA, int MB, long K) {
   for (; want; want /= 2) {
     try {
       s->get("rns_sum", sum);
-      s->get("mu_judge_counter", sizeof(RnsStats));  // "counter", "barrier": zeroed when allocated
+      s->get("mu_stats_counter", sizeof(RnsStats));  // "counter", "barrier": zeroed when allocated
       s->get("mu_sides_counter", sides);
       s->get("mu_tc_err_barrier", sizeof(int) * 4);
       s->get("rns_exp", p.exps * want);
@@ -685,8 +685,8 @@ int rns_reserve(Session *s, int MA, int MB, long K) {
 }
 
 // sum (hi + lo, MA x MB) = sum_k conj(A[i][k]) B[j][k], k < K (complex FP64 or FP32 rows of K), `slab`
-// chunks at a time (rns_reserve), and what it is to be judged by.
-RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab) {
+// chunks at a time (rns_reserve), and what it is to be checked by.
+RnsSum zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int MB, long K, bool fp32_inputs, int slab) {
   const RnsPlan p = rns_plan(MA, MB, K);
   const int kc = p.kc, nkb = kc / kBk, pitch = (MB + 15) / 16 * 16;
   double2 *sum_hi = (double2 *)s->get("rns_sum", sizeof(double2) * 2 * (size_t)MA * MB);
@@ -696,7 +696,7 @@ RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int 
   uint8_t *res = (uint8_t *)s->get("rns_res", p.res * slab);
   int *eA = (int *)s->get("rns_exp", p.exps * slab);
   int *eB = eA + (size_t)MA * slab;
-  RnsStats *stats = (RnsStats *)s->get("mu_judge_counter", sizeof(RnsStats));
+  RnsStats *stats = (RnsStats *)s->get("mu_stats_counter", sizeof(RnsStats));
   RnsSide *side = (RnsSide *)s->get("mu_sides_counter", sizeof(RnsSide) * 2 * (size_t)p.chunks);
   int *err = (int *)s->get("mu_tc_err_barrier", sizeof(int) * 4);  // read by mu_tc_check_error
   s->barrier_used = true;
@@ -738,7 +738,7 @@ RnsJudgement zgemm_cn_rns(Session *s, const void *A, int MA, const void *B, int 
 
 // After a wait that expired: the statistics of the contractions so far are void.
 void rns_clear_stats(Session *s) {
-  for (const char *name : {"mu_judge_counter", "mu_sides_counter", "mu_tiles_counter"}) {
+  for (const char *name : {"mu_stats_counter", "mu_sides_counter", "mu_tiles_counter"}) {
     auto it = s->ws.find(name);
     if (it != s->ws.end()) LQ_CUDA(cudaMemsetAsync(it->second.first, 0, it->second.second, s->stream));
   }

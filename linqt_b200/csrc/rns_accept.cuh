@@ -1,5 +1,5 @@
 // Acceptance of a contraction in residues (mu_rns.cu), which gathers the statistics; mu_gemm.cu
-// judges by them and commits the sum or the FP64 kernel's.
+// checks by them and commits the sum or the FP64 kernel's.
 #pragma once
 
 #include "internal.cuh"
@@ -8,7 +8,7 @@ namespace linqt {
 
 constexpr int kMaxParts = 8;  // parts of a row chunk (k_residues)
 
-// What the acceptance of a contraction is judged by, zero between contractions (the last block of
+// What the acceptance of a contraction is decided by, zero between contractions (the last block of
 // k_commit clears it).  Maxima are taken on the bits of non-negative doubles, whose order is
 // that of the numbers: the same in any order of arrival.
 struct RnsSide {
@@ -36,7 +36,7 @@ __device__ __forceinline__ void raise_to(unsigned long long *a, double v) {
 // |b| by (ua |b| (+) ub |a|) / sqrt(6), (+) and the chunks in quadrature; the largest of the rows
 // stand for all.  By one warp of a CTA, through L1: with every warp of a few hundred CTAs reading these few
 // lines from L2, their one slice took 10 to 20 us.  Not finite: rejected.
-__device__ __forceinline__ bool judge(const RnsSide *side, int nchunk, double top, double accept) {
+__device__ __forceinline__ bool rns_rejected(const RnsSide *side, int nchunk, double top, double accept) {
   const double allowed = accept * top;
   double sum = 0.0;
   for (int c = threadIdx.x & 31; c < nchunk; c += 32) {
